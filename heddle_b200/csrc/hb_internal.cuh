@@ -348,12 +348,12 @@ struct hb_forcefield {
                                      // build, [2] running count of a build,
                                      // [3] largest candidate count seen
   uint32_t *h_status = nullptr;      // pinned mirror
-  int pair_blocks_per_sm = 8;        // persistent pair kernel residency (tunable)
-  int pair_chunk = 4;                // packed entries per pair work item (tunable)
+  int pair_blocks_per_sm = 0;        // persistent pair kernel residency (tunable; 0: by form)
+  int pair_chunk = 0;                // packed entries per pair work item (tunable; 0: by size)
   int pair_quota = 0;                // work items per pair warp (0: persistent; tunable)
   uint32_t nl_polls = 1u << 20;      // poll limit of the tile build's bounded waits
   uint32_t nl_issue = 1;             // 0 (test only): issue no bulk copies, so the waits run out
-  uint32_t *d_work = nullptr;        // work counter of the balanced pair kernel
+  uint32_t *d_work = nullptr;        // work counter of the pair kernel
                                      // (zeroed by the combine kernel)
   uint64_t rebuilds_host = 0;
   bool built = false;

@@ -11,11 +11,12 @@
 //     r_search of a tile, which is 10% less pair-kernel work);
 //   * all per-step force work runs in this sorted-slot space (positions are
 //     gathered once per step, forces are scattered back once);
-//   * one block per i-tile sweeps j-tiles J > I through an AABB prune, keeps
-//     every j-atom within r_search of any i-atom, and deals them round-robin
-//     into entries of 32 together with a 32-bit exclusion mask per j-atom
-//     (bit m: the pair with i-atom m is in the exclusion list), so the pair
-//     kernel never scans exclusion lists for ordinary pairs;
+//   * one block per i-tile sweeps the j-tiles whose pair it owns through an
+//     AABB prune, keeps every j-atom within r_search of any i-atom, and deals
+//     them round-robin into entries of 32 together with a 32-bit exclusion
+//     mask per j-atom (bit m: the pair with i-atom m is in the exclusion
+//     list), so the pair kernel never scans exclusion lists for ordinary
+//     pairs;
 //   * the self tile is entry 0 of each i-tile and is evaluated with a half
 //     rotation (each unordered pair once);
 //   * entries live in a fixed-size slab per i-tile (sized from a counting
@@ -347,7 +348,7 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t k) {
 }
 
 // Packed-entry construction, one 256-thread block per i-tile I:
-//  1. the block sweeps j-tiles J > I in order, keeping those whose box lies
+//  1. the block sweeps its j-tiles in order, keeping those whose box lies
 //     within r_search of I's box (candidate list in shared memory);
 //  2. each warp takes candidates and computes a 32-bit hit mask: bit l is
 //     set when j-atom l of the candidate lies within r_search of any i-atom.
@@ -401,7 +402,6 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
   // step (warp w takes the w-th run of them, its lanes one 32-tile group
   // after another, so the list stays in tile order)
   auto box_near = [&](uint32_t J) {
-    if (J >= n_tiles) return false;
     if (!ortho) return true;
     const float4 cj = center[J], hj = half[J];
     float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
@@ -411,13 +411,21 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
     const float ez = fmaxf(fabsf(dz) - (hi.z + hj.z), 0.0f);
     return ex * ex + ey * ey + ez * ez <= rb2;
   };
-  for (uint32_t base = I + 1u; base < n_tiles; base += 32u * NLT_SWEEP * NLT_WARPS) {
+  // a tile pair belongs to its lower tile when the two numbers add up to an
+  // even one and to its higher tile otherwise: a tile's own share of its
+  // surroundings is then spread over all directions, which evens out its
+  // i-atoms' pairs (the lanes of the pair kernel) and the tiles' entries
+  const uint32_t n_below = (I + 1u) >> 1, n_mine = n_below + (n_tiles - 1u - I) / 2u;
+  auto tile_of = [&](uint32_t q) {
+    return q < n_below ? ((I + 1u) & 1u) + 2u * q : I + 2u + 2u * (q - n_below);
+  };
+  for (uint32_t base = 0u; base < n_mine; base += 32u * NLT_SWEEP * NLT_WARPS) {
     const uint32_t J0 = base + w * 32u * NLT_SWEEP + lane;
     uint32_t bal[NLT_SWEEP];
     uint32_t tot = 0u;
 #pragma unroll
     for (int q = 0; q < NLT_SWEEP; ++q) {
-      bal[q] = __ballot_sync(0xFFFFFFFFu, box_near(J0 + 32u * q));
+      bal[q] = __ballot_sync(0xFFFFFFFFu, J0 + 32u * q < n_mine && box_near(tile_of(J0 + 32u * q)));
       tot += __popc(bal[q]);
     }
     if (lane == 0) s_cnt[w] = tot;
@@ -429,7 +437,7 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
     for (int q = 0; q < NLT_SWEEP; ++q) {
       if ((bal[q] >> lane) & 1u) {
         const uint32_t pos = off + __popc(bal[q] & below);
-        if (pos < maxc) cand[pos] = J0 + 32u * q;
+        if (pos < maxc) cand[pos] = tile_of(J0 + 32u * q);
       }
       off += __popc(bal[q]);
     }
@@ -670,17 +678,8 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
       }
       const uint64_t slot = ((uint64_t)I * slab + e) * 32u + lane;
       entry_j[slot] = sj;
-      // stored in the i-lane's rotation order: bit t of lane l's word says
-      // whether i-atom l and the j-atom of lane (l + t) mod 32 are excluded
-      const uint32_t jm = excl_mask(sj, I, sorted_ids, inv_perm, eoff, epart);
-      uint32_t im = 0u;
-      if (__any_sync(0xFFFFFFFFu, jm != 0u)) {
-        for (uint32_t t = 0; t < 32u; ++t) {
-          const uint32_t m = __shfl_sync(0xFFFFFFFFu, jm, (lane + t) & 31u);
-          im |= ((m >> lane) & 1u) << t;
-        }
-      }
-      entry_excl[slot] = im;
+      // bit i of a j-atom's word: excluded with i-atom i of the tile
+      entry_excl[slot] = excl_mask(sj, I, sorted_ids, inv_perm, eoff, epart);
     }
   }
   if (threadIdx.x == 0) {
