@@ -102,6 +102,28 @@ __device__ __forceinline__ void hb_min_image(float &dx, float &dy, float &dz,
   dz -= kc * b.lz;
 }
 
+// periodic form of a tile's pairs: j-atoms already shifted next to the tile
+// (single periodic copy), orthorhombic minimum image, general minimum image
+enum { HB_IMAGE_NONE = 0, HB_IMAGE_ORTHO = 1, HB_IMAGE_TILTED = 2 };
+
+// minimum image of two separations at once
+template <int FORM>
+__device__ __forceinline__ void hb_min_image2(float2 &dx, float2 &dy, float2 &dz, const DBox &b) {
+  if constexpr (FORM == HB_IMAGE_ORTHO) {
+    // round(d / L) by adding and taking away 1.5 x 2^23 (|d| <= L here)
+    const float2 m = make_float2(12582912.0f, 12582912.0f), nm = make_float2(-12582912.0f, -12582912.0f);
+    const float2 kx = __fadd2_rn(__ffma2_rn(dx, make_float2(b.ilx, b.ilx), m), nm);
+    const float2 ky = __fadd2_rn(__ffma2_rn(dy, make_float2(b.ily, b.ily), m), nm);
+    const float2 kz = __fadd2_rn(__ffma2_rn(dz, make_float2(b.ilz, b.ilz), m), nm);
+    dx = __ffma2_rn(kx, make_float2(-b.lx, -b.lx), dx);
+    dy = __ffma2_rn(ky, make_float2(-b.ly, -b.ly), dy);
+    dz = __ffma2_rn(kz, make_float2(-b.lz, -b.lz), dz);
+  } else if constexpr (FORM == HB_IMAGE_TILTED) {
+    hb_min_image(dx.x, dy.x, dz.x, b);
+    hb_min_image(dx.y, dy.y, dz.y, b);
+  }
+}
+
 // wrap into the primary cell [-1/2, 1/2)^3 (fractional) and return the
 // image triple (kernels/pbc.cuh:73-91 semantics)
 __device__ __forceinline__ void hb_wrap(float &x, float &y, float &z, int &ka,

@@ -22,13 +22,12 @@
 //   * entries live in a fixed-size slab per i-tile (sized from a counting
 //     pass at the first build), so a rebuild is one pass and the layout is
 //     identical run to run;
-//   * a j-atom is refined against the 32 i-atoms only when it lies within
-//     r_search of the i-tile's box (one test prunes most far atoms);
 //   * every rebuild kernel is gated on the device status word, so a rebuild
 //     is decided on the device each step with no host read.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "hb_internal.cuh"
 
@@ -269,45 +268,76 @@ __global__ void k_tile_fill(const uint32_t *gate, uint32_t *sorted_ids,
 // rebuild: half + r_skin / 2 + rc_max <= L / 2 on every axis of an
 // orthorhombic box (the condition of jit_composed.rs:1577-1607 with the
 // skin margin added, because atoms drift between rebuilds).
-__global__ void k_tile_bbox(const uint32_t *gate, const float4 *__restrict__ tile_posq,
-                            const DBox *__restrict__ box, float rc_max, float r_skin,
-                            float4 *__restrict__ center, float4 *__restrict__ half, uint32_t n,
-                            uint32_t n_tiles) {
+// One block per 32 consecutive tiles; their common box follows the tiles'
+// (entries n_tiles + group of the two arrays).
+__global__ void __launch_bounds__(1024)
+    k_tile_bbox(const uint32_t *gate, const float4 *__restrict__ tile_posq,
+                const DBox *__restrict__ box, float rc_max, float r_skin,
+                float4 *__restrict__ center, float4 *__restrict__ half, uint32_t n,
+                uint32_t n_tiles) {
   if (gate_off(gate)) return;
-  uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  uint32_t lane = threadIdx.x & 31u;
-  if (warp >= n_tiles) return;
-  uint32_t k = warp * 32u + lane;
-  bool valid = k < n;
-  float4 p = tile_posq[k];
+  __shared__ float s_lo[3][32], s_hi[3][32];
+  const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t tile = blockIdx.x * 32u + w;
+  const uint32_t k = tile * 32u + lane;
+  const bool valid = tile < n_tiles && k < n;
+  const float4 p = valid ? tile_posq[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float lo[3] = {valid ? p.x : 3.0e38f, valid ? p.y : 3.0e38f, valid ? p.z : 3.0e38f};
   float hi[3] = {valid ? p.x : -3.0e38f, valid ? p.y : -3.0e38f, valid ? p.z : -3.0e38f};
+  auto reduce = [&]() {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], o));
+      }
+    }
+  };
+  auto store = [&](uint32_t at, float flags) {
+    center[at] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), flags);
+    half[at] = make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.0f);
+  };
+  reduce();
+  if (lane == 0) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], o));
-      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], o));
+      s_lo[d][w] = lo[d];
+      s_hi[d][w] = hi[d];
+    }
+    if (tile < n_tiles) {
+      const DBox b = *box;
+      float h[3];
+      for (int d = 0; d < 3; ++d) h[d] = 0.5f * (hi[d] - lo[d]);
+      // the margin also covers a cell scaled by up to HB_BOX_SLACK before the
+      // next rebuild (atoms move by up to that fraction of the half width)
+      const float m = 0.5f * r_skin + rc_max;
+      const float hw = 0.5f - HB_BOX_SLACK;
+      const bool spc = b.ortho && (h[0] + m <= hw * b.lx) && (h[1] + m <= hw * b.ly) &&
+                       (h[2] + m <= hw * b.lz);
+      // bit 0: single periodic copy; bit 1: per-axis minimum-image box tests
+      // are exact (orthorhombic cell)
+      store(tile, (float)((spc ? 1 : 0) | (b.ortho ? 2 : 0)));
     }
   }
-  if (lane == 0) {
-    DBox b = *box;
-    float c[3], h[3];
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      c[d] = 0.5f * (lo[d] + hi[d]);
-      h[d] = 0.5f * (hi[d] - lo[d]);
+      lo[d] = s_lo[d][lane];
+      hi[d] = s_hi[d][lane];
     }
-    // the margin also covers a cell scaled by up to HB_BOX_SLACK before the
-    // next rebuild (atoms move by up to that fraction of the half width)
-    float m = 0.5f * r_skin + rc_max;
-    const float hw = 0.5f - HB_BOX_SLACK;
-    bool spc = b.ortho && (h[0] + m <= hw * b.lx) && (h[1] + m <= hw * b.ly) &&
-               (h[2] + m <= hw * b.lz);
-    // bit 0: single periodic copy; bit 1: per-axis minimum-image box tests
-    // are exact (orthorhombic cell)
-    const int flags = (spc ? 1 : 0) | (b.ortho ? 2 : 0);
-    center[warp] = make_float4(c[0], c[1], c[2], (float)flags);
-    half[warp] = make_float4(h[0], h[1], h[2], 0.0f);
+    reduce();
+    if (lane == 0) {
+      // half a unit in the last place of the tiles' own boxes
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float g = 1.0e-6f * (fabsf(lo[d]) + fabsf(hi[d]));
+        lo[d] -= g;
+        hi[d] += g;
+      }
+      store(n_tiles + blockIdx.x, 0.0f);
+    }
   }
 }
 
@@ -329,7 +359,11 @@ __device__ __forceinline__ uint32_t excl_mask(uint32_t sj, uint32_t I,
 }
 
 #define NLT_WARPS 8
-#define NLT_SWEEP 4  // 32-tile groups per warp and block step of the candidate sweep
+#define NLT_SWEEP 4  // 32-lane ballots per warp and block step of the candidate sweep
+// candidate sweep by boxes of 32 tiles first: from this many tiles, and up
+// to this many near groups
+#define NLT_GROUPS_FROM 512u
+#define NLT_GROUPS 256u
 
 // k-th set bit (0-based) of a 32-bit mask
 // (k < popc(m)), by a binary search on the popcounts of low halves
@@ -352,12 +386,10 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t k) {
 //     within r_search of I's box (candidate list in shared memory);
 //  2. each warp takes candidates and computes a 32-bit hit mask: bit l is
 //     set when j-atom l of the candidate lies within r_search of any i-atom.
-//     Far from the r_search boundary a j-atom shifted once to the image
-//     nearest I's centre decides with plain differences; inside a 1e-4
-//     relative band the exact single-precision rule decides.  With the
-//     single shift, only the j-atoms within r_search of one of the i-tile's
-//     8-atom sub-tile boxes are refined, one at a time, with the lanes as
-//     i-atoms and one vote per j-atom;
+//     Far from the r_search boundary plain differences decide (of the
+//     j-atom shifted once to the image nearest I's centre, where the cell
+//     allows it); inside a 1e-4 relative band the exact single-precision
+//     rule decides;
 //  3. a prefix sum of the masks' popcounts fixes where every hit goes;
 //  4. the warps write the entries (self tile first) into I's slab, each
 //     with the exclusion masks of its 32 j-atoms.
@@ -380,7 +412,9 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
   uint32_t *pre = hmask + maxc;       // [maxc + 1] exclusive prefix of hits
   __shared__ uint32_t s_cnt[NLT_WARPS];
   __shared__ uint32_t s_ncand;
-  __shared__ float4 s_jsh[NLT_WARPS][32], s_jor[NLT_WARPS][32];  // a candidate's j-atoms: shifted, as stored
+  __shared__ float4 s_ixy[16];  // i-atoms 2k, 2k + 1: (x, x', y, y')
+  __shared__ float2 s_iz[16];   // (z, z')
+  __shared__ uint32_t s_group[NLT_GROUPS], s_ngroup;
   // per warp, two candidate tiles in flight: bulk copies (TMA engine) fill
   // one buffer while the warp refines the other
   __shared__ __align__(128) float4 s_jt[NLT_WARPS][2][32];
@@ -391,41 +425,54 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
   const float4 ci = center[I], hi = half[I];
   const bool ortho = ((int)ci.w & 2) != 0;
   const float rb2 = rb * rb;
-  // corner distance^2 below which a sub-tile's atoms all lie inside the
-  // plain-hit band (a relative margin far above the rounding of the boxes
-  // and of the distances)
-  const float acc2 = band_lo * (1.0f - 1.0e-5f);
   if (threadIdx.x == 0) s_ncand = 0u;
+  // the i-atoms in pairs for the packed refinement (a padding slot repeats
+  // the tile's first atom, which changes no minimum)
+  if (threadIdx.x < 32u) {
+    const float4 p = tile_posq[I * 32u + (I * 32u + threadIdx.x < n ? threadIdx.x : 0u)];
+    float *q = reinterpret_cast<float *>(&s_ixy[threadIdx.x >> 1]);
+    q[threadIdx.x & 1u] = p.x;
+    q[2u + (threadIdx.x & 1u)] = p.y;
+    reinterpret_cast<float *>(&s_iz[threadIdx.x >> 1])[threadIdx.x & 1u] = p.z;
+  }
   __syncthreads();
 
-  // 1. ordered candidate sweep, NLT_SWEEP x 32 tiles per warp per block
-  // step (warp w takes the w-th run of them, its lanes one 32-tile group
-  // after another, so the list stays in tile order)
-  auto box_near = [&](uint32_t J) {
-    if (!ortho) return true;
-    const float4 cj = center[J], hj = half[J];
+  // 1. ordered candidate sweep.  Orthorhombic cells: the gap between the two
+  // boxes at the nearest image.  Other cells: no image of the box centres is
+  // nearer than their distance along a cell face's normal, so a pair of
+  // tiles is out when that exceeds r_search plus the boxes' half diagonals
+  float wa = 0.0f, wb = 0.0f, ri = 0.0f;
+  if (!ortho) {
+    const float bay = -b.xy * b.ilx * b.ily, baz = (b.xy * b.yz - b.xz * b.ly) * b.ilx * b.ily * b.ilz;
+    const float bbz = -b.yz * b.ily * b.ilz;
+    wa = rsqrtf(b.ilx * b.ilx + bay * bay + baz * baz);
+    wb = rsqrtf(b.ily * b.ily + bbz * bbz);
+    ri = sqrtf(hi.x * hi.x + hi.y * hi.y + hi.z * hi.z);
+  }
+  auto boxes_near = [&](const float4 &cj, const float4 &hj) {
     float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+    if (!ortho) {
+      float sa, sb, sc;
+      hb_frac(dx, dy, dz, b, sa, sb, sc);
+      const float reach = (rb + ri + sqrtf(hj.x * hj.x + hj.y * hj.y + hj.z * hj.z)) * (1.0f + 1.0e-4f);
+      return fabsf(sa - rintf(sa)) * wa <= reach && fabsf(sb - rintf(sb)) * wb <= reach &&
+             fabsf(sc - rintf(sc)) * b.lz <= reach;
+    }
     hb_min_image(dx, dy, dz, b);
     const float ex = fmaxf(fabsf(dx) - (hi.x + hj.x), 0.0f);
     const float ey = fmaxf(fabsf(dy) - (hi.y + hj.y), 0.0f);
     const float ez = fmaxf(fabsf(dz) - (hi.z + hj.z), 0.0f);
     return ex * ex + ey * ey + ez * ez <= rb2;
   };
-  // a tile pair belongs to its lower tile when the two numbers add up to an
-  // even one and to its higher tile otherwise: a tile's own share of its
-  // surroundings is then spread over all directions, which evens out its
-  // i-atoms' pairs (the lanes of the pair kernel) and the tiles' entries
-  const uint32_t n_below = (I + 1u) >> 1, n_mine = n_below + (n_tiles - 1u - I) / 2u;
-  auto tile_of = [&](uint32_t q) {
-    return q < n_below ? ((I + 1u) & 1u) + 2u * q : I + 2u + 2u * (q - n_below);
-  };
-  for (uint32_t base = 0u; base < n_mine; base += 32u * NLT_SWEEP * NLT_WARPS) {
-    const uint32_t J0 = base + w * 32u * NLT_SWEEP + lane;
-    uint32_t bal[NLT_SWEEP];
+  // appends the candidates among J = first + 32 q + lane (q < NLT_SWEEP, one
+  // run of tiles per warp in tile order) to the block's list
+  auto append = [&](auto owned) {
+    uint32_t bal[NLT_SWEEP], J[NLT_SWEEP];
     uint32_t tot = 0u;
 #pragma unroll
     for (int q = 0; q < NLT_SWEEP; ++q) {
-      bal[q] = __ballot_sync(0xFFFFFFFFu, J0 + 32u * q < n_mine && box_near(tile_of(J0 + 32u * q)));
+      J[q] = owned(q);
+      bal[q] = __ballot_sync(0xFFFFFFFFu, J[q] < n_tiles && boxes_near(center[J[q]], half[J[q]]));
       tot += __popc(bal[q]);
     }
     if (lane == 0) s_cnt[w] = tot;
@@ -437,7 +484,7 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
     for (int q = 0; q < NLT_SWEEP; ++q) {
       if ((bal[q] >> lane) & 1u) {
         const uint32_t pos = off + __popc(bal[q] & below);
-        if (pos < maxc) cand[pos] = tile_of(J0 + 32u * q);
+        if (pos < maxc) cand[pos] = J[q];
       }
       off += __popc(bal[q]);
     }
@@ -448,44 +495,90 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
       s_ncand = t;
     }
     __syncthreads();
+  };
+  // a tile pair belongs to its lower tile when the two numbers add up to an
+  // even one and to its higher tile otherwise: a tile's own share of its
+  // surroundings is then spread over all directions, which evens out its
+  // i-atoms' pairs (the lanes of the pair kernel) and the tiles' entries
+  bool grouped = false;
+  const uint32_t n_groups = (n_tiles + 31u) / 32u;
+  if (n_tiles >= NLT_GROUPS_FROM) {
+    // many tiles: boxes of 32 consecutive tiles (compact runs of the Hilbert
+    // curve) first, then the tiles of the near ones
+    if (threadIdx.x == 0) s_ngroup = 0u;
+    for (uint32_t base = 0u; base < n_groups; base += 32u * NLT_WARPS) {
+      const uint32_t G = base + threadIdx.x;
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, G < n_groups && boxes_near(center[n_tiles + G], half[n_tiles + G]));
+      if (lane == 0) s_cnt[w] = __popc(bal);
+      __syncthreads();
+      uint32_t off = s_ngroup;
+      for (uint32_t k = 0; k < w; ++k) off += s_cnt[k];
+      if ((bal >> lane) & 1u) {
+        const uint32_t pos = off + __popc(bal & ((1u << lane) - 1u));
+        if (pos < NLT_GROUPS) s_group[pos] = G;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (uint32_t k = 0; k < NLT_WARPS; ++k) s_ngroup += s_cnt[k];
+      __syncthreads();
+    }
+    grouped = s_ngroup <= NLT_GROUPS;
+  }
+  if (grouped) {
+    // lanes 0-15 and 16-31 take the owned half of one near group each
+    const uint32_t n_near = s_ngroup;
+    for (uint32_t base = 0u; base < n_near; base += 2u * NLT_SWEEP * NLT_WARPS) {
+      append([&](int q) {
+        const uint32_t k = base + (w * NLT_SWEEP + (uint32_t)q) * 2u + (lane >> 4);
+        if (k >= n_near) return 0xFFFFFFFFu;
+        // tiles below I: odd distance; above: even
+        const uint32_t J0 = s_group[k] * 32u, t = (lane & 15u) * 2u, par = I & 1u;
+        const uint32_t lo = J0 + t + (par ^ 1u), up = J0 + t + par;  // J0 is even
+        if (J0 + 32u <= I) return lo;
+        if (J0 > I) return up;
+        // I's own group: both kinds; the owned tile of each pair of tiles
+        return lo < I ? lo : (up > I ? up : 0xFFFFFFFFu);
+      });
+    }
+  } else {
+    const uint32_t n_below = (I + 1u) >> 1, n_mine = n_below + (n_tiles - 1u - I) / 2u;
+    for (uint32_t base = 0u; base < n_mine; base += 32u * NLT_SWEEP * NLT_WARPS) {
+      append([&](int q) {
+        const uint32_t k = base + w * 32u * NLT_SWEEP + 32u * (uint32_t)q + lane;
+        if (k >= n_mine) return 0xFFFFFFFFu;
+        return k < n_below ? ((I + 1u) & 1u) + 2u * k : I + 2u + 2u * (k - n_below);
+      });
+    }
   }
   const uint32_t ncand_all = s_ncand;
   const uint32_t ncand = ncand_all < maxc ? ncand_all : maxc;
 
-  // 2. hit masks; i-atoms stay in registers and are broadcast by shuffles
+  // 2. hit masks: one lane per j-atom of the candidate, its smallest
+  // distance to the tile's i-atoms over broadcast pairs of them in the packed
+  // FP32x2 pipe (plain distances only decide far from the band, so their
+  // rounding is free)
   const uint32_t ki = I * 32u + lane;
-  const float4 pim = tile_posq[ki];
-  const uint32_t ivalid = __ballot_sync(0xFFFFFFFFu, ki < n);
+  const uint32_t n_i = min(n - I * 32u, 32u);
   const bool shift_ok = ortho && (hi.x + rb <= 0.5f * b.lx) && (hi.y + rb <= 0.5f * b.ly) &&
                         (hi.z + rb <= 0.5f * b.lz);
-  // With the single shift, the tile's four 8-atom sub-tiles (lanes 8q..8q+7)
-  // get their own boxes: a j-atom is refined only against the atoms of the
-  // sub-tiles whose box lies within r_search (plus the rounding margin), so
-  // a j-atom near one corner of the tile costs 8 or 16 tests instead of 32.
-  // Every pair within r_search lies in the box of its i-atom's sub-tile, so
-  // the hits are those of the full refinement.
-  float sc[4][3], sh[4][3];
-  if (shift_ok) {
-    const bool iv = ki < n;
-    float lo3[3] = {iv ? pim.x : 3.0e38f, iv ? pim.y : 3.0e38f, iv ? pim.z : 3.0e38f};
-    float hi3[3] = {iv ? pim.x : -3.0e38f, iv ? pim.y : -3.0e38f, iv ? pim.z : -3.0e38f};
+  auto nearest2 = [&](auto form, float x, float y, float z) {
+    constexpr int FORM = decltype(form)::value;
+    const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
+    float best = 3.0e38f;
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo3[d] = fminf(lo3[d], __shfl_xor_sync(0xFFFFFFFFu, lo3[d], o));
-        hi3[d] = fmaxf(hi3[d], __shfl_xor_sync(0xFFFFFFFFu, hi3[d], o));
-      }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float l = __shfl_sync(0xFFFFFFFFu, lo3[d], 8 * q);
-        const float h = __shfl_sync(0xFFFFFFFFu, hi3[d], 8 * q);
-        sc[q][d] = 0.5f * (l + h);
-        sh[q][d] = h >= l ? 0.5f * (h - l) : -1.0f;  // empty sub-tile: never near
-      }
-  }
+    for (int k = 0; k < 16; ++k) {
+      const float4 a = s_ixy[k];
+      float2 dx = __fadd2_rn(make_float2(a.x, a.y), nx);
+      float2 dy = __fadd2_rn(make_float2(a.z, a.w), ny);
+      float2 dz = __fadd2_rn(s_iz[k], nz);
+      hb_min_image2<FORM>(dx, dy, dz, b);
+      float2 r2 = __fmul2_rn(dx, dx);
+      r2 = __ffma2_rn(dy, dy, r2);
+      r2 = __ffma2_rn(dz, dz, r2);
+      best = fminf(best, fminf(r2.x, r2.y));
+    }
+    return best;
+  };
   // candidate tiles are staged by bulk copies one candidate ahead; a wait
   // that runs out sets HB_ST_DEVICE_TIMEOUT (the host returns
   // HB_ERR_DEVICE_TIMEOUT), drains the copies still in flight and stops
@@ -524,96 +617,16 @@ __global__ void __launch_bounds__(NLT_WARPS * 32, 4)
       sy -= b.ly * rintf((sy - ci.y) * b.ily);
       sz -= b.lz * rintf((sz - ci.z) * b.ilz);
     }
-    if (shift_ok) {
-      uint32_t qm = 0u;
-      bool inside = false;
-      if (jvalid) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float ax = fabsf(sx - sc[q][0]), ay = fabsf(sy - sc[q][1]),
-                      az = fabsf(sz - sc[q][2]);
-          const float ex = fmaxf(ax - sh[q][0], 0.0f);
-          const float ey = fmaxf(ay - sh[q][1], 0.0f);
-          const float ez = fmaxf(az - sh[q][2], 0.0f);
-          if (sh[q][0] >= 0.0f && ex * ex + ey * ey + ez * ez <= rb2) qm |= 1u << q;
-          // the box's farthest corner well inside the band: every i-atom of
-          // the (non-empty) sub-tile is, so the vote would find a plain hit
-          const float fx = ax + sh[q][0], fy = ay + sh[q][1], fz = az + sh[q][2];
-          if (sh[q][0] >= 0.0f && fx * fx + fy * fy + fz * fz < acc2) inside = true;
-        }
+    const float r2 = shift_ok ? nearest2(std::integral_constant<int, HB_IMAGE_NONE>{}, sx, sy, sz)
+                     : ortho  ? nearest2(std::integral_constant<int, HB_IMAGE_ORTHO>{}, sx, sy, sz)
+                              : nearest2(std::integral_constant<int, HB_IMAGE_TILTED>{}, sx, sy, sz);
+    bool hit = jvalid && r2 < band_lo;
+    if (jvalid && !hit && r2 <= band_hi) {
+      // in the band: the exact rule on the stored positions
+      for (uint32_t m = 0; m < n_i && !hit; ++m) {
+        const float4 pi = tile_posq[I * 32u + m];
+        hit = hb_exact_r2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z, b) <= rs2;
       }
-      // the j-atoms near a sub-tile box are refined one at a time with the
-      // lanes as i-atoms: each lane tests its own i-atom against the
-      // broadcast j-atom and one vote decides (padding i-slots sit at 1e18
-      // and never hit); the exact rule runs only when some pair falls in
-      // the band.  The j-atoms found inside a sub-tile's reach above need
-      // no vote.
-      const uint32_t sure = __ballot_sync(0xFFFFFFFFu, inside);
-      uint32_t rem = __ballot_sync(0xFFFFFFFFu, qm != 0u && !inside);
-      s_jsh[w][lane] = make_float4(sx, sy, sz, 0.0f);
-      s_jor[w][lane] = pj;
-      __syncwarp();
-      // two near j-atoms per step in the packed FP32x2 pipe (plain
-      // distances only decide far from the band, so their rounding is free)
-      uint32_t hm = sure;
-      const float2 px2 = make_float2(pim.x, pim.x), py2 = make_float2(pim.y, pim.y),
-                   pz2 = make_float2(pim.z, pim.z);
-      auto vote = [&](uint32_t jl, float r2) {
-        bool hit = __any_sync(0xFFFFFFFFu, r2 < band_lo);
-        const bool inb = r2 >= band_lo && r2 <= band_hi;
-        if (!hit && __any_sync(0xFFFFFFFFu, inb)) {
-          const float4 qo = s_jor[w][jl];
-          const bool ex = inb && hb_exact_r2(pim.x - qo.x, pim.y - qo.y, pim.z - qo.z, b) <= rs2;
-          hit = __any_sync(0xFFFFFFFFu, ex);
-        }
-        if (hit) hm |= 1u << jl;
-      };
-      while (rem != 0u) {
-        const uint32_t ja = (uint32_t)__ffs(rem) - 1u;
-        rem &= rem - 1u;
-        const bool two = rem != 0u;
-        const uint32_t jb = two ? (uint32_t)__ffs(rem) - 1u : ja;
-        rem &= rem - 1u;
-        const float4 qa = s_jsh[w][ja], qb = s_jsh[w][jb];
-        const float2 dx = __fadd2_rn(px2, make_float2(-qa.x, -qb.x));
-        const float2 dy = __fadd2_rn(py2, make_float2(-qa.y, -qb.y));
-        const float2 dz = __fadd2_rn(pz2, make_float2(-qa.z, -qb.z));
-        float2 r2 = __fmul2_rn(dx, dx);
-        r2 = __ffma2_rn(dy, dy, r2);
-        r2 = __ffma2_rn(dz, dz, r2);
-        vote(ja, r2.x);
-        if (two) vote(jb, r2.y);
-      }
-      __syncwarp();
-      if (lane == 0) hmask[c] = hm;
-      continue;
-    }
-    bool near = jvalid;
-    if (near && ortho) {
-      float dx = sx - ci.x, dy = sy - ci.y, dz = sz - ci.z;
-      hb_min_image(dx, dy, dz, b);
-      const float ex = fmaxf(fabsf(dx) - hi.x, 0.0f);
-      const float ey = fmaxf(fabsf(dy) - hi.y, 0.0f);
-      const float ez = fmaxf(fabsf(dz) - hi.z, 0.0f);
-      near = ex * ex + ey * ey + ez * ez <= rb2;
-    }
-    bool hit = false;
-    uint32_t open = __ballot_sync(0xFFFFFFFFu, near);
-    for (uint32_t m = 0; m < 32u && open != 0u; ++m) {
-      const float xi = __shfl_sync(0xFFFFFFFFu, pim.x, m);
-      const float yi = __shfl_sync(0xFFFFFFFFu, pim.y, m);
-      const float zi = __shfl_sync(0xFFFFFFFFu, pim.z, m);
-      if (near && !hit && ((ivalid >> m) & 1u)) {
-        float dx = xi - sx, dy = yi - sy, dz = zi - sz;
-        hb_min_image(dx, dy, dz, b);
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 < band_lo) {
-          hit = true;
-        } else if (r2 <= band_hi && hb_exact_r2(xi - pj.x, yi - pj.y, zi - pj.z, b) <= rs2) {
-          hit = true;
-        }
-      }
-      open = __ballot_sync(0xFFFFFFFFu, near && !hit);
     }
     const uint32_t hm = __ballot_sync(0xFFFFFFFFu, hit);
     if (lane == 0) hmask[c] = hm;
@@ -778,8 +791,10 @@ int nl_setup(hb_forcefield *ff) {
   HB_CUDA(cudaMalloc(&ff->d_inv_perm, sizeof(uint32_t) * std::max(n, 1u)));
   HB_CUDA(cudaMalloc(&ff->d_tile_posq, sizeof(float4) * n_pad));
   HB_CUDA(cudaMalloc(&ff->d_tile_type, sizeof(int) * n_pad));
-  HB_CUDA(cudaMalloc(&ff->d_tile_center, sizeof(float4) * std::max(ff->n_tiles, 1u)));
-  HB_CUDA(cudaMalloc(&ff->d_tile_half, sizeof(float4) * std::max(ff->n_tiles, 1u)));
+  // tiles, then groups of 32 tiles
+  const uint32_t n_boxes = std::max(ff->n_tiles, 1u) + hb_div_up(std::max(ff->n_tiles, 1u), 32);
+  HB_CUDA(cudaMalloc(&ff->d_tile_center, sizeof(float4) * n_boxes));
+  HB_CUDA(cudaMalloc(&ff->d_tile_half, sizeof(float4) * n_boxes));
   HB_CUDA(cudaMalloc(&ff->d_tile_nent, sizeof(uint32_t) * (ff->n_tiles + 1)));
   HB_CUDA(cudaMemset(ff->d_tile_nent, 0, sizeof(uint32_t) * (ff->n_tiles + 1)));
   HB_CUDA(cudaMalloc(&ff->d_ref_pos, sizeof(float4) * std::max(n, 1u)));
@@ -846,7 +861,7 @@ static int nl_launch(hb_forcefield *ff, const uint32_t *gate, cudaStream_t s, bo
     k_tile_fill<<<hb_div_up(ff->n_pad, 256), 256, 0, s>>>(
         gate, ff->d_sorted_ids, sys->d_posq, sys->d_image, ff->d_inv_perm, ff->d_tile_posq,
         ff->d_tile_type, ff->d_ref_pos, n, ff->n_pad);
-    k_tile_bbox<<<hb_div_up((uint64_t)ff->n_tiles * 32u, 128), 128, 0, s>>>(
+    k_tile_bbox<<<hb_div_up(ff->n_tiles, 32), 1024, 0, s>>>(
         gate, ff->d_tile_posq, sys->d_box, ff->rc_max, ff->r_skin, ff->d_tile_center,
         ff->d_tile_half, n, ff->n_tiles);
   }

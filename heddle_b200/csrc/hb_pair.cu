@@ -122,10 +122,6 @@ __device__ __forceinline__ void red_add(unsigned long long *p, long long v) {
 #define PK_ESCALE 268435456.0f    // 2^28
 #define PK_EMAX 0.25f
 
-// periodic form of a tile's pairs: j-atoms already shifted next to the tile
-// (single periodic copy), orthorhombic minimum image, general minimum image
-enum { PF_SINGLE = 0, PF_ORTHO = 1, PF_TILTED = 2 };
-
 template <bool EV, bool SCALED, bool EXACT>
 struct PairWarp {
   using acc_t = typename std::conditional<EXACT, unsigned long long, int>::type;
@@ -165,24 +161,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-
-// minimum image of two separations at once
-template <int FORM>
-__device__ __forceinline__ void min_image2(float2 &dx, float2 &dy, float2 &dz, const DBox &b) {
-  if constexpr (FORM == PF_ORTHO) {
-    // round(d / L) by adding and taking away 1.5 x 2^23 (|d| <= L here)
-    const float2 m = make_float2(12582912.0f, 12582912.0f), nm = make_float2(-12582912.0f, -12582912.0f);
-    const float2 kx = __fadd2_rn(__ffma2_rn(dx, make_float2(b.ilx, b.ilx), m), nm);
-    const float2 ky = __fadd2_rn(__ffma2_rn(dy, make_float2(b.ily, b.ily), m), nm);
-    const float2 kz = __fadd2_rn(__ffma2_rn(dz, make_float2(b.ilz, b.ilz), m), nm);
-    dx = __ffma2_rn(kx, make_float2(-b.lx, -b.lx), dx);
-    dy = __ffma2_rn(ky, make_float2(-b.ly, -b.ly), dy);
-    dz = __ffma2_rn(kz, make_float2(-b.lz, -b.lz), dz);
-  } else if constexpr (FORM == PF_TILTED) {
-    hb_min_image(dx.x, dy.x, dz.x, b);
-    hb_min_image(dx.y, dy.y, dz.y, b);
-  }
 }
 
 template <bool EV, bool SCALED, bool SWITCH, bool EXACT, bool MULTI>
@@ -324,7 +302,7 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
     auto item = [&](auto form) {
       constexpr int FORM = decltype(form)::value;
       if (!ivalid) pi = make_float4(-1.0e18f, -1.0e18f, -1.0e18f, 0.0f);
-      else if (FORM == PF_SINGLE) shift_to(pi.x, pi.y, pi.z, c, b);
+      else if (FORM == HB_IMAGE_NONE) shift_to(pi.x, pi.y, pi.z, c, b);
       // the entry whose data the prefetch registers hold goes to rows
       // [base, base + 32); returns the lane's hits, a bound on the mask of its
       // hits without a Lennard-Jones term, and (SCALED) its listed exclusions
@@ -334,7 +312,7 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
         float4 pj = pj_n;
         const int tj = tj_n;
         const bool jvalid = sj != HB_SENTINEL;
-        if (FORM == PF_SINGLE && jvalid) shift_to(pj.x, pj.y, pj.z, c, b);
+        if (FORM == HB_IMAGE_NONE && jvalid) shift_to(pj.x, pj.y, pj.z, c, b);
         const bool jl = jvalid && (few_types ? ((any_lj >> tj) & 1u) != 0u : any_lj != 0u);
         const uint32_t b_v = __ballot_sync(0xFFFFFFFFu, jvalid), b_l = __ballot_sync(0xFFFFFFFFu, jl);
         const uint32_t n_v = __popc(b_v), n_l = __popc(b_l);
@@ -382,7 +360,7 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
           float2 dx = __fadd2_rn(px, make_float2(a.x, a.y));
           float2 dy = __fadd2_rn(py, make_float2(a.z, a.w));
           float2 dz = __fadd2_rn(pz, S.jz2[k]);
-          min_image2<FORM>(dx, dy, dz, b);
+          hb_min_image2<FORM>(dx, dy, dz, b);
           float2 r2 = __fmul2_rn(dx, dx);
           r2 = __ffma2_rn(dy, dy, r2);
           r2 = __ffma2_rn(dz, dz, r2);
@@ -446,7 +424,7 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
             float2 dx = make_float2(pi.x - ja.x, pi.x - jb.x);
             float2 dy = make_float2(pi.y - ja.y, pi.y - jb.y);
             float2 dz = make_float2(pi.z - ja.z, pi.z - jb.z);
-            min_image2<FORM>(dx, dy, dz, b);
+            hb_min_image2<FORM>(dx, dy, dz, b);
             float2 r2 = __fmul2_rn(dx, dx);
             r2 = __ffma2_rn(dy, dy, r2);
             r2 = __ffma2_rn(dz, dz, r2);
@@ -707,9 +685,9 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
       }
     };
     const int flags = (int)c.w;
-    if (!EXACT && (flags & 1) != 0) item(std::integral_constant<int, PF_SINGLE>{});
-    else if ((flags & 2) != 0) item(std::integral_constant<int, PF_ORTHO>{});
-    else item(std::integral_constant<int, PF_TILTED>{});
+    if (!EXACT && (flags & 1) != 0) item(std::integral_constant<int, HB_IMAGE_NONE>{});
+    else if ((flags & 2) != 0) item(std::integral_constant<int, HB_IMAGE_ORTHO>{});
+    else item(std::integral_constant<int, HB_IMAGE_TILTED>{});
     if (ivalid) {
       red_add(&fp[0 * np_all + si], ax);
       red_add(&fp[1 * np_all + si], ay);
