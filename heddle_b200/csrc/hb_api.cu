@@ -1659,10 +1659,11 @@ extern "C" int hb_integrator_count_launches(hb_integrator *it, hb_forcefield *ff
   if (it->baro && it->sys->n) HB_TRY(count_captured(it, ff, cons, false, true, eager_move));
   // in the graph form the gated rebuild kernels move into the IF node's
   // body and one kernel sets the condition
-  const uint64_t body = ff->sys->n ? (uint64_t)nl_kernel_count() : 0u;
-  kernels[0] = eager - body + (body ? 1u : 0u);
+  const uint64_t body = ff->sys->n ? (uint64_t)nl_kernel_count(ff, false) : 0u;
+  const uint64_t gated = ff->sys->n ? (uint64_t)nl_kernel_count(ff, true) : 0u;
+  kernels[0] = eager - gated + (body ? 1u : 0u);
   kernels[1] = body;
-  kernels[2] = eager_move ? eager_move - body + 1u : 0u;
+  kernels[2] = eager_move ? eager_move - gated + 1u : 0u;
   return HB_OK;
 }
 

@@ -345,6 +345,7 @@ struct hb_forcefield {
   uint32_t n_tiles = 0, n_pad = 0;
   int nv_log2 = 5;                 // voxel grid 2^nv_log2 per axis
   uint32_t *d_vox_key = nullptr;   // per atom
+  uint32_t *d_vox_rank = nullptr;    // an atom's place within its voxel (cluster sort)
   uint32_t *d_vox_count = nullptr; // per voxel (+1)
   uint32_t *d_vox_off = nullptr;
   uint32_t *d_scan_tmp = nullptr;
@@ -560,7 +561,7 @@ int nl_free(hb_forcefield *ff);
 // Rebuild the list.  gated: kernels run only when the status word has the
 // displacement bit set (a device-side decision, no host read).
 int nl_rebuild(hb_forcefield *ff, bool gated, cudaStream_t s);
-int nl_kernel_count();
+int nl_kernel_count(const hb_forcefield *ff, bool eager);
 // During stream capture: the rebuild as a device-side conditional graph node.
 int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s);
 int nl_displacement_check(hb_forcefield *ff, cudaStream_t s);

@@ -107,15 +107,7 @@ __device__ __forceinline__ uint32_t hilbert_key(uint32_t x, uint32_t y, uint32_t
   return h;
 }
 
-__global__ void k_vox_hist(const uint32_t *gate, const float4 *__restrict__ posq,
-                           const DBox *__restrict__ box, int nv_log2,
-                           uint32_t *__restrict__ key, uint32_t *__restrict__ count,
-                           uint32_t n) {
-  if (gate_off(gate)) return;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  DBox b = *box;
-  float4 p = posq[i];
+__device__ __forceinline__ uint32_t voxel_of(const float4 &p, const DBox &b, int nv_log2) {
   float sa, sb, sc;
   hb_frac(p.x, p.y, p.z, b, sa, sb, sc);
   const int nv = 1 << nv_log2;
@@ -127,7 +119,17 @@ __global__ void k_vox_hist(const uint32_t *gate, const float4 *__restrict__ posq
     int c = (int)(u * (float)nv);
     v[d] = c < 0 ? 0 : (c >= nv ? nv - 1 : c);
   }
-  const uint32_t k = hilbert_key((uint32_t)v[0], (uint32_t)v[1], (uint32_t)v[2], nv_log2);
+  return hilbert_key((uint32_t)v[0], (uint32_t)v[1], (uint32_t)v[2], nv_log2);
+}
+
+__global__ void k_vox_hist(const uint32_t *gate, const float4 *__restrict__ posq,
+                           const DBox *__restrict__ box, int nv_log2,
+                           uint32_t *__restrict__ key, uint32_t *__restrict__ count,
+                           uint32_t n) {
+  if (gate_off(gate)) return;
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t k = voxel_of(posq[i], *box, nv_log2);
   key[i] = k;
   atomicAdd(&count[k], 1u);
 }
@@ -268,20 +270,16 @@ __global__ void k_tile_fill(const uint32_t *gate, uint32_t *sorted_ids,
 // rebuild: half + r_skin / 2 + rc_max <= L / 2 on every axis of an
 // orthorhombic box (the condition of jit_composed.rs:1577-1607 with the
 // skin margin added, because atoms drift between rebuilds).
-// One block per 32 consecutive tiles; their common box follows the tiles'
+// A block of 32 warps takes 32 consecutive tiles; their common box follows the tiles'
 // (entries n_tiles + group of the two arrays).
-__global__ void __launch_bounds__(1024)
-    k_tile_bbox(const uint32_t *gate, const float4 *__restrict__ tile_posq,
-                const DBox *__restrict__ box, float rc_max, float r_skin,
-                float4 *__restrict__ center, float4 *__restrict__ half, uint32_t n,
-                uint32_t n_tiles) {
-  if (gate_off(gate)) return;
-  __shared__ float s_lo[3][32], s_hi[3][32];
+__device__ __forceinline__ void tile_boxes(uint32_t group, float4 p, const DBox *__restrict__ box,
+                                           float rc_max, float r_skin, float4 *__restrict__ center,
+                                           float4 *__restrict__ half, uint32_t n, uint32_t n_tiles,
+                                           float (*s_lo)[32], float (*s_hi)[32]) {
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t tile = blockIdx.x * 32u + w;
+  const uint32_t tile = group * 32u + w;
   const uint32_t k = tile * 32u + lane;
   const bool valid = tile < n_tiles && k < n;
-  const float4 p = valid ? tile_posq[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float lo[3] = {valid ? p.x : 3.0e38f, valid ? p.y : 3.0e38f, valid ? p.z : 3.0e38f};
   float hi[3] = {valid ? p.x : -3.0e38f, valid ? p.y : -3.0e38f, valid ? p.z : -3.0e38f};
   auto reduce = [&]() {
@@ -336,8 +334,128 @@ __global__ void __launch_bounds__(1024)
         lo[d] -= g;
         hi[d] += g;
       }
-      store(n_tiles + blockIdx.x, 0.0f);
+      store(n_tiles + group, 0.0f);
     }
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(1024)
+    k_tile_bbox(const uint32_t *gate, const float4 *__restrict__ tile_posq,
+                const DBox *__restrict__ box, float rc_max, float r_skin,
+                float4 *__restrict__ center, float4 *__restrict__ half, uint32_t n,
+                uint32_t n_tiles) {
+  if (gate_off(gate)) return;
+  __shared__ float s_lo[3][32], s_hi[3][32];
+  const uint32_t k = blockIdx.x * 1024u + threadIdx.x;
+  const float4 p = k < n ? tile_posq[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  tile_boxes(blockIdx.x, p, box, rc_max, r_skin, center, half, n, n_tiles, s_lo, s_hi);
+}
+
+// ---------------------------------------------------------------------
+// The whole sort of a rebuild -- histogram, scan, scatter, order by id, slot
+// views, boxes -- as one kernel of one thread-block cluster, whose barriers
+// take the place of seven kernel boundaries.  Each thread keeps its atoms'
+// rank from the histogram's atomics, so the scatter needs no second pass of
+// them.  See nl_launch for where it is used.
+// ---------------------------------------------------------------------
+#define NLS_CTAS 8
+#define NLS_MAX_ATOMS 24576u
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(NLS_CTAS, 1, 1) __launch_bounds__(1024)
+    k_nl_sort(const uint32_t *gate, const float4 *__restrict__ posq, const int4 *__restrict__ image,
+              const DBox *__restrict__ box, int nv_log2, uint32_t *key, uint32_t *rank,
+              uint32_t *count, uint32_t *off, uint32_t *totals, uint32_t *sorted_ids,
+              uint32_t *__restrict__ inv_perm, float4 *__restrict__ tile_posq,
+              int *__restrict__ tile_type, float4 *__restrict__ ref_pos, float rc_max, float r_skin,
+              float4 *__restrict__ center, float4 *__restrict__ half, uint32_t n, uint32_t n_tiles) {
+  if (gate_off(gate)) return;  // the same answer in every block of the cluster
+  __shared__ uint32_t ws[32];
+  __shared__ float s_lo[3][32], s_hi[3][32];
+  constexpr uint32_t T = NLS_CTAS * 1024u;
+  const uint32_t t = blockIdx.x * 1024u + threadIdx.x;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const uint32_t n_vox = 1u << (3 * nv_log2);
+  const DBox b = *box;
+  for (uint32_t i = t; i < n; i += T) {
+    const uint32_t k = voxel_of(posq[i], b, nv_log2);
+    key[i] = k;
+    rank[i] = atomicAdd(&count[k], 1u);
+  }
+  cluster_sync();
+  // exclusive scan: a run of `per` voxels per thread (the counts were left in
+  // L2 by the atomics), warps and blocks in order
+  const uint32_t per = (n_vox + T - 1u) / T, v0 = t * per;
+  uint32_t sum = 0u;
+  for (uint32_t q = 0; q < per; ++q)
+    if (v0 + q < n_vox) sum += __ldcg(&count[v0 + q]);
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    if ((int)lane >= o) x += y;
+  }
+  if (lane == 31u) ws[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    uint32_t y = ws[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t z = __shfl_up_sync(0xFFFFFFFFu, y, o);
+      if ((int)lane >= o) y += z;
+    }
+    ws[lane] = y;
+    if (lane == 31u) __stcg(&totals[blockIdx.x], y);
+  }
+  cluster_sync();
+  uint32_t base = x - sum + (w > 0 ? ws[w - 1] : 0u);
+  for (uint32_t q = 0; q < blockIdx.x; ++q) base += __ldcg(&totals[q]);
+  for (uint32_t q = 0; q < per; ++q) {
+    const uint32_t v = v0 + q;
+    if (v < n_vox) {
+      const uint32_t c = __ldcg(&count[v]);
+      off[v] = base;
+      base += c;
+      count[v] = 0u;  // for the next rebuild
+      if (v == n_vox - 1u) off[n_vox] = base;
+    }
+  }
+  cluster_sync();
+  for (uint32_t i = t; i < n; i += T) sorted_ids[__ldcg(&off[key[i]]) + rank[i]] = i;
+  cluster_sync();
+  for (uint32_t v = t; v < n_vox; v += T) {
+    const uint32_t s = __ldcg(&off[v]), e = __ldcg(&off[v + 1]);
+    for (uint32_t k = s + 1; k < e; ++k) {
+      const uint32_t id = __ldcg(&sorted_ids[k]);
+      int p = (int)k - 1;
+      while (p >= (int)s && __ldcg(&sorted_ids[p]) > id) {
+        __stcg(&sorted_ids[p + 1], __ldcg(&sorted_ids[p]));
+        --p;
+      }
+      __stcg(&sorted_ids[p + 1], id);
+    }
+  }
+  cluster_sync();
+  const uint32_t n_pad = n_tiles * 32u, n_groups = (n_tiles + 31u) / 32u;
+  for (uint32_t g = blockIdx.x; g < n_groups; g += NLS_CTAS) {
+    const uint32_t k = g * 1024u + threadIdx.x;
+    float4 p = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.0f);
+    if (k < n) {
+      const uint32_t id = __ldcg(&sorted_ids[k]);
+      inv_perm[id] = k;
+      p = posq[id];
+      tile_type[k] = image[id].w;
+      ref_pos[id] = p;
+    } else if (k < n_pad) {
+      sorted_ids[k] = HB_SENTINEL;
+      tile_type[k] = 0;
+    }
+    if (k < n_pad) tile_posq[k] = p;
+    tile_boxes(g, p, box, rc_max, r_skin, center, half, n, n_tiles, s_lo, s_hi);
   }
 }
 
@@ -782,11 +900,12 @@ int nl_setup(hb_forcefield *ff) {
   const uint32_t n_vox = 1u << (3 * l2);
   const uint32_t n_pad = ff->n_pad ? ff->n_pad : 32u;
   HB_CUDA(cudaMalloc(&ff->d_vox_key, sizeof(uint32_t) * std::max(n, 1u)));
+  HB_CUDA(cudaMalloc(&ff->d_vox_rank, sizeof(uint32_t) * std::max(n, 1u)));
   HB_CUDA(cudaMalloc(&ff->d_vox_count, sizeof(uint32_t) * (n_vox + 1)));
   HB_CUDA(cudaMemset(ff->d_vox_count, 0, sizeof(uint32_t) * (n_vox + 1)));
   HB_CUDA(cudaMalloc(&ff->d_vox_off, sizeof(uint32_t) * (n_vox + 1)));
   uint32_t scan_len = std::max(n_vox + 1, ff->n_tiles + 1);
-  HB_CUDA(cudaMalloc(&ff->d_scan_tmp, sizeof(uint32_t) * (hb_div_up(scan_len, 1024) + 1)));
+  HB_CUDA(cudaMalloc(&ff->d_scan_tmp, sizeof(uint32_t) * std::max<uint32_t>(hb_div_up(scan_len, 1024) + 1, NLS_CTAS)));
   HB_CUDA(cudaMalloc(&ff->d_sorted_ids, sizeof(uint32_t) * n_pad));
   HB_CUDA(cudaMalloc(&ff->d_inv_perm, sizeof(uint32_t) * std::max(n, 1u)));
   HB_CUDA(cudaMalloc(&ff->d_tile_posq, sizeof(float4) * n_pad));
@@ -814,6 +933,7 @@ int nl_setup(hb_forcefield *ff) {
 
 int nl_free(hb_forcefield *ff) {
   cudaFree(ff->d_vox_key);
+  cudaFree(ff->d_vox_rank);
   cudaFree(ff->d_vox_count);
   cudaFree(ff->d_vox_off);
   cudaFree(ff->d_scan_tmp);
@@ -836,11 +956,22 @@ int nl_free(hb_forcefield *ff) {
   return HB_OK;
 }
 
+// Whether an eager rebuild sorts in one cluster kernel.  Every eager force
+// evaluation launches the rebuild's kernels, gated off by the status word in
+// most: eight fewer launches take a gated-off check from 76-78 to 50 us at
+// any size, and a forced rebuild from 93 to 77 us at 1,029 atoms and from 104
+// to 90 us at 6,000.  Above some 25,000 atoms (131 against 136 us) one
+// cluster is too few SMs for the work itself (65,856 atoms: 172 against
+// 310 us).  In a graph the kernels are an IF node's body, which costs nothing
+// when it is not taken.
+static bool nl_one_sort(const hb_forcefield *ff) { return ff->sys->n <= NLS_MAX_ATOMS; }
+
 // The rebuild sequence: voxel sort, sorted-slot views and tile boxes
 // (sort), then either the counting pass of the first build (count_only)
-// or the single fill pass plus the finishing kernel.
+// or the fill pass plus the finishing kernel.  `eager`: launched one by one,
+// not as the body of a graph's IF node.
 static int nl_launch(hb_forcefield *ff, const uint32_t *gate, cudaStream_t s, bool sort,
-                     bool count_only) {
+                     bool count_only, bool eager) {
   hb_system *sys = ff->sys;
   const uint32_t n = sys->n;
   const uint32_t n_vox = 1u << (3 * ff->nv_log2);
@@ -851,7 +982,13 @@ static int nl_launch(hb_forcefield *ff, const uint32_t *gate, cudaStream_t s, bo
   const float rb = rs * (1.0f + 1.0e-4f) + 1.0e-4f;
   const float band_lo = rs2 * (1.0f - 1.0e-4f), band_hi = rs2 * (1.0f + 1.0e-4f);
   const size_t smem = sizeof(uint32_t) * (3u * ff->maxc + 1u);
-  if (sort) {
+  if (sort && eager && nl_one_sort(ff)) {
+    k_nl_sort<<<NLS_CTAS, 1024, 0, s>>>(
+        gate, sys->d_posq, sys->d_image, sys->d_box, ff->nv_log2, ff->d_vox_key, ff->d_vox_rank,
+        ff->d_vox_count, ff->d_vox_off, ff->d_scan_tmp, ff->d_sorted_ids, ff->d_inv_perm,
+        ff->d_tile_posq, ff->d_tile_type, ff->d_ref_pos, ff->rc_max, ff->r_skin,
+        ff->d_tile_center, ff->d_tile_half, n, ff->n_tiles);
+  } else if (sort) {
     k_vox_hist<<<hb_div_up(n, 256), 256, 0, s>>>(gate, sys->d_posq, sys->d_box, ff->nv_log2,
                                                   ff->d_vox_key, ff->d_vox_count, n);
     HB_TRY(scan_exclusive(gate, ff->d_vox_count, ff->d_vox_off, ff->d_scan_tmp, n_vox + 1, s));
@@ -884,19 +1021,20 @@ static int nl_launch(hb_forcefield *ff, const uint32_t *gate, cudaStream_t s, bo
 }
 
 // kernels launched by one rebuild: voxel histogram, three scan kernels,
-// scatter, voxel sort, tile fill, tile boxes, tile build, finish
-int nl_kernel_count() { return 10; }
+// scatter, voxel sort, tile fill and tile boxes (or, eager, the cluster
+// sort), tile build, finish
+int nl_kernel_count(const hb_forcefield *ff, bool eager) { return eager && nl_one_sort(ff) ? 3 : 10; }
 
 int nl_rebuild(hb_forcefield *ff, bool gated, cudaStream_t s) {
   if (ff->sys->n == 0) return HB_OK;
   const uint32_t *gate = gated ? ff->d_status : nullptr;
   if (!gated) {
-    // an explicit rebuild: raise the displacement bit so k_nl_finish clears it
+    // an explicit rebuild: raise the displacement bit, which its end clears
     uint32_t one = HB_ST_DISPLACED;
     HB_CUDA(cudaMemcpyAsync(ff->d_status, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     HB_CUDA(cudaStreamSynchronize(s));
   }
-  return nl_launch(ff, gate, s, true, false);
+  return nl_launch(ff, gate, s, true, false, true);
 }
 
 // First build: counting pass, slab size = 1.5 x the largest tile count + 4,
@@ -913,7 +1051,7 @@ int nl_first_build(hb_forcefield *ff) {
   HB_CUDA(cudaMemcpyAsync(ff->d_status, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   for (int attempt = 0; attempt < 4; ++attempt) {
     HB_CUDA(cudaMemsetAsync(ff->d_counters + 3, 0, sizeof(uint32_t), s));
-    HB_TRY(nl_launch(ff, nullptr, s, attempt == 0, true));
+    HB_TRY(nl_launch(ff, nullptr, s, attempt == 0, true, true));
     uint32_t mc = 0;
     HB_CUDA(cudaMemcpyAsync(&mc, ff->d_counters + 3, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     HB_CUDA(cudaStreamSynchronize(s));
@@ -946,7 +1084,7 @@ int nl_first_build(hb_forcefield *ff) {
     ff->entry_cap = cap;
     ff->layout_gen++;
   }
-  HB_TRY(nl_launch(ff, nullptr, s, false, false));
+  HB_TRY(nl_launch(ff, nullptr, s, false, false, true));
   uint32_t st = 0;
   HB_CUDA(cudaMemcpyAsync(&st, ff->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   HB_CUDA(cudaStreamSynchronize(s));
@@ -1022,7 +1160,7 @@ int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s) {
   cudaStream_t side = ff->sys->ctx->stream3;
   HB_CUDA(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal));
-  int rc = nl_launch(ff, nullptr, side, true, false);
+  int rc = nl_launch(ff, nullptr, side, true, false, false);
   cudaGraph_t out;
   cudaError_t ce = cudaStreamEndCapture(side, &out);
   if (rc != HB_OK) return rc;
