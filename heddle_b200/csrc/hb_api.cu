@@ -665,10 +665,7 @@ static int force_pre(hb_forcefield *ff, bool ev, bool capturing) {
   hb_context *ctx = ff->sys->ctx;
   cudaStream_t s = ctx->stream, s2 = ctx->stream2;
   cudaEvent_t t0 = stage_begin(s);
-  HB_TRY(nl_displacement_check(ff, s));
-  if (capturing) HB_TRY(nl_rebuild_conditional(ff, s));
-  else HB_TRY(nl_rebuild(ff, true, s));
-  HB_TRY(nl_gather_positions(ff, s));
+  HB_TRY(nl_update(ff, capturing, s));
   stage_end(3, t0, s);
   // bonded terms add into the same fixed-point accumulators (slots of the
   // current list), before the pair kernel on the main stream
@@ -1657,13 +1654,13 @@ extern "C" int hb_integrator_count_launches(hb_integrator *it, hb_forcefield *ff
   uint64_t eager = 0, eager_move = 0;
   HB_TRY(count_captured(it, ff, cons, true, false, eager));
   if (it->baro && it->sys->n) HB_TRY(count_captured(it, ff, cons, false, true, eager_move));
-  // in the graph form the gated rebuild kernels move into the IF node's
-  // body and one kernel sets the condition
+  // in the graph form the rebuild kernels move into the IF node's body (the
+  // displacement check sets its condition)
   const uint64_t body = ff->sys->n ? (uint64_t)nl_kernel_count(ff, false) : 0u;
   const uint64_t gated = ff->sys->n ? (uint64_t)nl_kernel_count(ff, true) : 0u;
-  kernels[0] = eager - gated + (body ? 1u : 0u);
+  kernels[0] = eager - gated;
   kernels[1] = body;
-  kernels[2] = eager_move ? eager_move - gated + 1u : 0u;
+  kernels[2] = eager_move ? eager_move - gated : 0u;
   return HB_OK;
 }
 

@@ -369,7 +369,8 @@ struct hb_forcefield {
   uint32_t *d_status = nullptr;      // status word
   uint32_t *d_counters = nullptr;    // [0] rebuilds, [1] entries of the last
                                      // build, [2] running count of a build,
-                                     // [3] largest candidate count seen
+                                     // [3] largest candidate count seen, [4]
+                                     // blocks done of the displacement check
   uint32_t *h_status = nullptr;      // pinned mirror
   int pair_blocks_per_sm = 0;        // persistent pair kernel residency (tunable; 0: by form)
   int pair_chunk = 0;                // packed entries per pair work item (tunable; 0: by size)
@@ -563,9 +564,8 @@ int nl_free(hb_forcefield *ff);
 int nl_rebuild(hb_forcefield *ff, bool gated, cudaStream_t s);
 int nl_kernel_count(const hb_forcefield *ff, bool eager);
 // During stream capture: the rebuild as a device-side conditional graph node.
-int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s);
 int nl_displacement_check(hb_forcefield *ff, cudaStream_t s);
-int nl_gather_positions(hb_forcefield *ff, cudaStream_t s);
+int nl_update(hb_forcefield *ff, bool capturing, cudaStream_t s);
 int nl_first_build(hb_forcefield *ff);
 int nl_set_slab(hb_forcefield *ff, uint32_t slab);
 int nl_pairs(hb_forcefield *ff, std::vector<uint32_t> &pairs, uint64_t &dups);

@@ -845,9 +845,17 @@ __global__ void k_nl_finish(const uint32_t *gate, uint32_t *status, uint32_t *co
 // atom's displacement d becomes min(r_skin, mu (r_c + r_skin) - r_c) / 2.
 // Any other change of the cell (a shear, a larger scaling, set_box to a new
 // shape) invalidates the list.
+//
+// COPY: the kernel has read every position, so it also writes the tile-order
+// copy that the force kernels read (a rebuild after it writes its own).
+// GRAPH: the last block to finish sets the condition of the graph's rebuild
+// node.  Both take a kernel out of every step's serial chain.
+template <bool COPY, bool GRAPH>
 __global__ void k_disp_check(const float4 *__restrict__ posq, const float4 *__restrict__ ref,
                              const DBox *__restrict__ box, const DBox *__restrict__ ref_box,
-                             float r_skin, float rc_max, uint32_t *status, uint32_t n) {
+                             float r_skin, float rc_max, uint32_t *status, uint32_t n,
+                             const uint32_t *__restrict__ inv_perm, float4 *__restrict__ tile_posq,
+                             uint32_t *done, cudaGraphConditionalHandle node) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const DBox a = *box, r = *ref_box;
   const float mu = a.lx / r.lx;  // r.lx = 0 before the first build: not finite
@@ -859,14 +867,28 @@ __global__ void k_disp_check(const float4 *__restrict__ posq, const float4 *__re
   float thr = 0.5f * r_skin;
   if (mu < 1.0f) thr = fminf(thr, 0.5f * (mu * (rc_max + r_skin) - rc_max));
   bool moved = i == 0u && (!iso || !(thr > 0.0f));
+  float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (i < n && (COPY || iso)) p = posq[i];
+  if (COPY && i < n) tile_posq[inv_perm[i]] = p;
   if (i < n && iso) {
-    const float4 p = posq[i], q = ref[i];
+    const float4 q = ref[i];
     float dx = p.x - mu * q.x, dy = p.y - mu * q.y, dz = p.z - mu * q.z;
     hb_min_image(dx, dy, dz, a);
     moved = moved || dx * dx + dy * dy + dz * dz > thr * thr;
   }
   // one atomic per warp at most
   if (__any_sync(0xFFFFFFFFu, moved) && (threadIdx.x & 31u) == 0u) atomicOr(status, HB_ST_DISPLACED);
+  if constexpr (GRAPH) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(done, 1u) == gridDim.x - 1u) {
+        *done = 0u;
+        __threadfence();
+        cudaGraphSetConditional(node, (atomicOr(status, 0u) & HB_ST_DISPLACED) ? 1u : 0u);
+      }
+    }
+  }
 }
 
 __global__ void k_gather_pos(const uint32_t *__restrict__ sorted_ids,
@@ -921,10 +943,10 @@ int nl_setup(hb_forcefield *ff) {
   HB_CUDA(cudaMemset(ff->d_ref_box, 0, sizeof(DBox)));
   HB_CUDA(cudaMalloc(&ff->d_status, sizeof(uint32_t)));
   HB_CUDA(cudaMemset(ff->d_status, 0, sizeof(uint32_t)));
-  HB_CUDA(cudaMalloc(&ff->d_counters, sizeof(uint32_t) * 4));
+  HB_CUDA(cudaMalloc(&ff->d_counters, sizeof(uint32_t) * 5));
   HB_CUDA(cudaMalloc(&ff->d_work, sizeof(uint32_t)));
   HB_CUDA(cudaMemset(ff->d_work, 0, sizeof(uint32_t)));
-  HB_CUDA(cudaMemset(ff->d_counters, 0, sizeof(uint32_t) * 4));
+  HB_CUDA(cudaMemset(ff->d_counters, 0, sizeof(uint32_t) * 5));
   HB_CUDA(cudaMallocHost(&ff->h_status, sizeof(uint32_t) * 8));
   HB_CUDA(cudaMalloc(&ff->d_fp, sizeof(unsigned long long) * 5 * n_pad));
   HB_CUDA(cudaMemset(ff->d_fp, 0, sizeof(unsigned long long) * 5 * n_pad));
@@ -1126,17 +1148,33 @@ int nl_set_slab(hb_forcefield *ff, uint32_t slab) {
   return nl_rebuild(ff, false, s);
 }
 
-namespace {
-__global__ void k_set_rebuild_condition(cudaGraphConditionalHandle h, const uint32_t *status) {
-  cudaGraphSetConditional(h, ((*status) & HB_ST_DISPLACED) ? 1u : 0u);
+static int disp_check(hb_forcefield *ff, bool copy, const cudaGraphConditionalHandle *node, cudaStream_t s) {
+  hb_system *sys = ff->sys;
+  auto launch = [&](auto kernel) {
+    kernel<<<hb_div_up(sys->n, 256), 256, 0, s>>>(
+        sys->d_posq, ff->d_ref_pos, sys->d_box, ff->d_ref_box, ff->r_skin, ff->rc_max, ff->d_status,
+        sys->n, ff->d_inv_perm, ff->d_tile_posq, ff->d_counters + 4,
+        node ? *node : cudaGraphConditionalHandle{});
+  };
+  if (node) copy ? launch(k_disp_check<true, true>) : launch(k_disp_check<false, true>);
+  else copy ? launch(k_disp_check<true, false>) : launch(k_disp_check<false, false>);
+  HB_CUDA(cudaGetLastError());
+  return HB_OK;
 }
-}  // namespace
 
-// Inside a stream capture: the rebuild becomes an IF node of the graph
-// being captured, taken when the displacement bit is set.  The body (the
-// ungated rebuild sequence) is captured on the context's side stream.
-int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s) {
-  if (ff->sys->n == 0) return HB_OK;
+// Whether the displacement check of a force evaluation also writes the
+// tile-order positions (else k_gather_pos does, after the rebuild).  Without
+// a reciprocal part it does (10,000 argon atoms: 38.1 -> 36.5 us per graph
+// step).  With one, two streams fork right after the rebuild node then, and
+// the pair kernel often takes the SMs before the charge spreading: 92.2 us
+// per step of 8,192 waters with the copy kernel, 92.1 or 97.6 without.
+static bool nl_check_copies(const hb_forcefield *ff) { return !ff->spme.on; }
+
+// Inside a stream capture: displacement check, then the rebuild as an IF
+// node of the graph being captured, taken when the displacement bit is set.
+// The body (the ungated rebuild sequence) is captured on the context's side
+// stream.
+static int check_and_rebuild_graph(hb_forcefield *ff, cudaStream_t s) {
   cudaStreamCaptureStatus st;
   cudaGraph_t g;
   const cudaGraphNode_t *deps = nullptr;
@@ -1146,8 +1184,7 @@ int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s) {
     return hb_fail(HB_ERR_INVALID_ARGUMENT, "conditional rebuild needs an active capture");
   cudaGraphConditionalHandle h;
   HB_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-  k_set_rebuild_condition<<<1, 1, 0, s>>>(h, ff->d_status);
-  HB_CUDA(cudaGetLastError());
+  HB_TRY(disp_check(ff, nl_check_copies(ff), &h, s));
   HB_CUDA(cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &nd));
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
@@ -1170,20 +1207,24 @@ int nl_rebuild_conditional(hb_forcefield *ff, cudaStream_t s) {
 }
 
 int nl_displacement_check(hb_forcefield *ff, cudaStream_t s) {
-  hb_system *sys = ff->sys;
-  if (sys->n == 0) return HB_OK;
-  k_disp_check<<<hb_div_up(sys->n, 256), 256, 0, s>>>(sys->d_posq, ff->d_ref_pos, sys->d_box,
-                                                       ff->d_ref_box, ff->r_skin, ff->rc_max,
-                                                       ff->d_status, sys->n);
-  HB_CUDA(cudaGetLastError());
-  return HB_OK;
+  if (ff->sys->n == 0) return HB_OK;
+  return disp_check(ff, false, nullptr, s);
 }
 
-int nl_gather_positions(hb_forcefield *ff, cudaStream_t s) {
+// The list part of a force evaluation: displacement check, rebuild where it
+// asks for one, positions in tile order.
+int nl_update(hb_forcefield *ff, bool capturing, cudaStream_t s) {
   hb_system *sys = ff->sys;
   if (sys->n == 0) return HB_OK;
-  k_gather_pos<<<hb_div_up(sys->n, 256), 256, 0, s>>>(ff->d_sorted_ids, sys->d_posq,
-                                                       ff->d_tile_posq, sys->n);
+  if (capturing) {
+    HB_TRY(check_and_rebuild_graph(ff, s));
+  } else {
+    HB_TRY(disp_check(ff, nl_check_copies(ff), nullptr, s));
+    HB_TRY(nl_rebuild(ff, true, s));
+  }
+  if (!nl_check_copies(ff))
+    k_gather_pos<<<hb_div_up(sys->n, 256), 256, 0, s>>>(ff->d_sorted_ids, sys->d_posq,
+                                                         ff->d_tile_posq, sys->n);
   HB_CUDA(cudaGetLastError());
   return HB_OK;
 }
