@@ -309,6 +309,7 @@ struct SpmeState {
   float2 *d_tw = nullptr;                     // twiddles a | b | c
   double *d_part = nullptr;                   // energy / virial partials
   int n_part = 0;
+  int use_cube = 0;   // small cubes: the whole transform in one cluster
   int use_plane = 0;                          // kc-major planes + whole-plane pass
   int gather_c = 1;                           // orders 4, 8: thread per (atom, c offset)
   double *d_sums = nullptr;                   // [2] E_recip, W_recip

@@ -728,13 +728,16 @@ uint32_t pair_chunk_of(const hb_forcefield *ff) {
 }
 
 // Resident blocks per SM when the caller set none.  With a reciprocal part
-// one block fewer than fit, so that its chain on the other stream finds SM
-// room beside the persistent blocks: 65,536-water graph step 414 us at 6,
-// 392 at 5, 453 at 4 (8,192 waters: 101, 96, 102)
+// fewer than fit, so that its chain on the other stream finds SM room beside
+// the persistent blocks: one fewer where whole planes are transformed (graph
+// step of 65,536 waters 414, 392, 453 us at 6, 5, 4; of 8,192 97, 91, 98 us),
+// two fewer where five line passes have to find room (2,000 waters 69, 64,
+// 60 us; 21,952: 209, 204, 196 us)
 uint32_t pair_blocks_of(const hb_forcefield *ff, bool wide) {
   if (ff->pair_blocks_per_sm > 0) return (uint32_t)ff->pair_blocks_per_sm;
   const uint32_t fit = wide ? PAIR_MIN_BLOCKS(true, false, false) : PAIR_MIN_BLOCKS(false, false, false);
-  return ff->spme.on ? fit - 1u : fit;
+  if (!ff->spme.on) return fit;
+  return ff->spme.use_plane || wide ? fit - 1u : fit - 2u;
 }
 
 template <bool EV, bool SCALED, bool SWITCH, bool EXACT>

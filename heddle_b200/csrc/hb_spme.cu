@@ -35,10 +35,15 @@
 // influence function and both inverse transforms run in place on the plane
 // in shared memory (radix-16 and radix-8 stages).  Deterministic by
 // construction.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "hb_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -836,6 +841,251 @@ __global__ void __launch_bounds__(PLANE_THREADS) k_fft_plane(
   }
 }
 
+// ---------------------------------------------------------------------
+// Small cubes: the whole transform, convolution and inverse as one kernel of
+// one cluster of 8 CTAs.  A CTA holds a slab of a-planes in shared memory
+// (transforms along c, two real rows per complex line, and along b), then a
+// share of the (b, kc) columns gathered from all slabs through distributed
+// shared memory (along a: forward, influence function, inverse), then its
+// slab again.  Bound: latency -- each stage is one or two butterflies per
+// thread and a barrier; what it saves is five kernels' launches, tails and
+// global round trips.  256 threads and at most 64 registers, so that its
+// CTAs fit beside resident pair blocks.
+// ---------------------------------------------------------------------
+constexpr int CUBE_CTAS = 8, CUBE_THREADS = 384;
+
+__host__ __device__ constexpr int cube_planes(int n) { return (n + CUBE_CTAS - 1) / CUBE_CTAS; }
+__host__ __device__ constexpr int cube_cols(int n) { return (n * (n / 2 + 1) + CUBE_CTAS - 1) / CUBE_CTAS; }
+// complex elements of each of the two buffers (a slab, or a share of columns)
+__host__ __device__ constexpr int cube_buffer(int n) {
+  return cube_planes(n) * (n / 2 + 1) > cube_cols(n) ? cube_planes(n) * n * (n / 2 + 1) : cube_cols(n) * n;
+}
+__host__ __device__ constexpr size_t cube_smem(int n) { return sizeof(float2) * (2 * (size_t)cube_buffer(n) + n); }
+
+// i = q m + r of a thread's elements i = threadIdx.x + k CUBE_THREADS, kept
+// without a division per element
+struct CubeWalk {
+  int m, dq, dr, q, r;
+  __device__ __forceinline__ explicit CubeWalk(int m_)
+      : m(m_), dq(CUBE_THREADS / m_), dr(CUBE_THREADS % m_), q((int)threadIdx.x / m_),
+        r((int)threadIdx.x % m_) {}
+  __device__ __forceinline__ void next() {
+    q += dq;
+    r += dr;
+    if (r >= m) {
+      r -= m;
+      ++q;
+    }
+  }
+};
+
+// Stockham stages over `lines` lines of length N: element k of line l at
+// off(l) + k es.  FAST: consecutive threads take consecutive lines (strided
+// lines), else consecutive butterflies of a line.  Returns the result buffer.
+template <int N, bool INV, bool FAST, int S = 0, int NS = 1, class Off>
+__device__ __forceinline__ float2 *cube_stages(float2 *A, float2 *B, const float2 *tw, int lines, int es,
+                                               Off off) {
+  if constexpr (S == n_stages(N)) {
+    return A;
+  } else {
+    constexpr int P = stage_radix(N, S), M = N / P, TSTEP = N / (NS * P);
+    CubeWalk at(FAST ? max(lines, 1) : M);
+    for (int idx = threadIdx.x; idx < M * lines; idx += CUBE_THREADS, at.next()) {
+      const int l = FAST ? at.r : at.q, j = FAST ? at.q : at.r;
+      const int k = j % NS, o = off(l);
+      float2 v[P];
+#pragma unroll
+      for (int q = 0; q < P; ++q) v[q] = A[o + (j + q * M) * es];
+      if constexpr (NS > 1) {
+#pragma unroll
+        for (int q = 1; q < P; ++q) {
+          const float2 w = tw[q * k * TSTEP];
+          v[q] = INV ? cmulc(v[q], w) : cmul(v[q], w);
+        }
+      }
+      butterfly<P, INV>(v);
+      const int base = (j / NS) * NS * P + k;
+#pragma unroll
+      for (int q = 0; q < P; ++q) B[o + (base + q * NS) * es] = v[q];
+    }
+    __syncthreads();
+    return cube_stages<N, INV, FAST, S + 1, NS * P>(B, A, tw, lines, es, off);
+  }
+}
+
+template <int N, bool EV>
+__global__ void __cluster_dims__(CUBE_CTAS, 1, 1) __launch_bounds__(CUBE_THREADS, 2)
+    k_fft_cube(unsigned long long *__restrict__ rho, float *__restrict__ V,
+               const float2 *__restrict__ tw_g, const DBox *__restrict__ box,
+               const float *__restrict__ bfac, float alpha, double *__restrict__ part) {
+  constexpr int NCH = N / 2 + 1, NP = (N + 1) / 2, PL = cube_planes(N), CPC = cube_cols(N);
+  extern __shared__ float2 smc[];
+  __shared__ double red_e[CUBE_THREADS / 32], red_w[CUBE_THREADS / 32];
+  cg::cluster_group cl = cg::this_cluster();
+  float2 *X = smc, *Y = smc + cube_buffer(N), *tw = Y + cube_buffer(N);
+  const int rank = blockIdx.x;
+  const int a0 = rank * PL, planes = max(0, min(PL, N - a0));
+  for (int i = threadIdx.x; i < N; i += CUBE_THREADS) tw[i] = tw_g[i];
+
+  // charges: rows b and b + 1 of a plane become one complex line
+  unsigned long long *slab = rho + (size_t)a0 * N * N;
+  constexpr int U = 8;
+  for (int i0 = threadIdx.x; i0 < planes * N * N; i0 += CUBE_THREADS * U) {
+    long long v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * CUBE_THREADS;
+      v[u] = i < planes * N * N ? (long long)slab[i] : 0ll;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * CUBE_THREADS;
+      if (i < planes * N * N) {
+        const int a = i / (N * N), b = (i / N) % N, c = i % N;
+        slab[i] = 0ull;
+        reinterpret_cast<float *>(X)[2 * ((a * NP + b / 2) * N + c) + (b & 1)] =
+            (float)v[u] * (1.0f / HB_RHO_SCALE);
+      }
+    }
+  }
+  if (N & 1)
+    for (int i = threadIdx.x; i < planes * N; i += CUBE_THREADS)
+      reinterpret_cast<float *>(X)[2 * (((i / N) * NP + NP - 1) * N + i % N) + 1] = 0.0f;
+  __syncthreads();
+  float2 *R = cube_stages<N, false, false>(X, Y, tw, planes * NP, 1, [](int l) { return l * N; });
+  float2 *O = R == X ? Y : X;
+  for (int i = threadIdx.x; i < planes * N * NCH; i += CUBE_THREADS) {
+    const int a = i / (N * NCH), b = (i / NCH) % N, k = i % NCH;
+    const float2 *line = R + (a * NP + b / 2) * N;
+    const float2 p = line[k], m = line[k ? N - k : 0];
+    O[i] = (b & 1) ? make_float2(0.5f * (p.y + m.y), 0.5f * (m.x - p.x))
+                   : make_float2(0.5f * (p.x + m.x), 0.5f * (p.y - m.y));
+  }
+  __syncthreads();
+  auto b_line = [](int l) { return (l / NCH) * (N * NCH) + l % NCH; };
+  float2 *Z = R;
+  R = cube_stages<N, false, true>(O, Z, tw, planes * NCH, NCH, b_line);
+  O = R == O ? Z : O;
+
+  // columns: element (a, col) lies in slab a / PL
+  const int col0 = rank * CPC, cols = max(0, min(CPC, N * NCH - col0));
+  cl.sync();
+  {
+    // several remote reads in flight per thread
+    CubeWalk at(max(cols, 1));
+    for (int i0 = threadIdx.x; i0 < N * cols; i0 += CUBE_THREADS * U) {
+      float2 v[U];
+      int to[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u, at.next()) {
+        to[u] = i0 + u * CUBE_THREADS < N * cols ? at.q * CPC + at.r : -1;
+        if (to[u] >= 0) v[u] = cl.map_shared_rank(R, at.q / PL)[(at.q % PL) * (N * NCH) + col0 + at.r];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (to[u] >= 0) O[to[u]] = v[u];
+    }
+  }
+  cl.sync();
+  auto a_line = [](int l) { return l; };
+  float2 *T = cube_stages<N, false, true>(O, R, tw, cols, CPC, a_line);
+  const DBox bx = *box;
+  const float ilx = bx.ilx, ily = bx.ily, ilz = bx.ilz;
+  const float bax = ilx, bay = -bx.xy * ilx * ily, baz = (bx.xy * bx.yz - bx.xz * bx.ly) * ilx * ily * ilz;
+  const float bby = ily, bbz = -bx.yz * ily * ilz, bcz = ilz;
+  const float two_pi = 6.283185307179586f;
+  const float inv_vol = ilx * ily * ilz;
+  const float inv4a2 = 1.0f / (4.0f * alpha * alpha);
+  const float inv2a2 = 1.0f / (2.0f * alpha * alpha);
+  double e_acc = 0.0, w_acc = 0.0;
+  CubeWalk mode(max(cols, 1));
+  for (int i = threadIdx.x; i < N * cols; i += CUBE_THREADS, mode.next()) {
+    const int ka = mode.q, c = mode.r, kb = (col0 + c) / NCH, kc = (col0 + c) % NCH;
+    const float ma = (ka <= N / 2) ? (float)ka : (float)(ka - N);
+    const float mb = (kb <= N / 2) ? (float)kb : (float)(kb - N);
+    const float mc = (float)kc;
+    const float kx = two_pi * (ma * bax);
+    const float ky = two_pi * (ma * bay + mb * bby);
+    const float kz = two_pi * (ma * baz + mb * bbz + mc * bcz);
+    const float k2 = kx * kx + ky * ky + kz * kz;
+    float G = 0.0f, vf = 0.0f;
+    if (k2 > 0.0f) {
+      G = inv_vol * (12.566370614359172f / k2) * expf(-k2 * inv4a2) * bfac[ka] * bfac[N + kb] * bfac[2 * N + kc];
+      if constexpr (EV) vf = G * (1.0f - k2 * inv2a2);
+    }
+    float2 &x = T[ka * CPC + c];
+    if constexpr (EV) {
+      const double hw = (kc == 0 || ((N & 1) == 0 && 2 * kc == N)) ? 1.0 : 2.0;
+      const double x2 = (double)x.x * x.x + (double)x.y * x.y;
+      e_acc += hw * (double)G * x2;
+      w_acc += hw * (double)vf * x2;
+    }
+    x = make_float2(G * x.x, G * x.y);
+  }
+  if constexpr (EV) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      e_acc += __shfl_xor_sync(0xFFFFFFFFu, e_acc, o);
+      w_acc += __shfl_xor_sync(0xFFFFFFFFu, w_acc, o);
+    }
+    if ((threadIdx.x & 31u) == 0u) {
+      red_e[threadIdx.x >> 5] = e_acc;
+      red_w[threadIdx.x >> 5] = w_acc;
+    }
+  }
+  __syncthreads();
+  if (EV && threadIdx.x == 0) {
+    double e = 0.0, w = 0.0;
+    for (int k = 0; k < CUBE_THREADS / 32; ++k) {
+      e += red_e[k];
+      w += red_w[k];
+    }
+    part[2 * rank] = e;
+    part[2 * rank + 1] = w;
+  }
+  float2 *T2 = T == O ? R : O;
+  R = cube_stages<N, true, true>(T, T2, tw, cols, CPC, a_line);
+  O = R == T ? T2 : T;
+  cl.sync();
+  for (int i0 = threadIdx.x; i0 < planes * N * NCH; i0 += CUBE_THREADS * U) {
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * CUBE_THREADS, a = i / (N * NCH), col = i - a * (N * NCH), own = col / CPC;
+      if (i < planes * N * NCH) v[u] = cl.map_shared_rank(R, own)[(a0 + a) * CPC + col - own * CPC];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * CUBE_THREADS < planes * N * NCH) O[i0 + u * CUBE_THREADS] = v[u];
+  }
+  cl.sync();  // no CTA's memory is read by another after this
+  Z = R;
+  R = cube_stages<N, true, true>(O, Z, tw, planes * NCH, NCH, b_line);
+  O = R == O ? Z : O;
+  // two rows' half spectra make one complex line; the modes 0 and N / 2 of a
+  // real row count with their real parts
+  for (int i = threadIdx.x; i < planes * NP * N; i += CUBE_THREADS) {
+    const int l = i / N, k = i - l * N, a = l / NP, b = 2 * (l % NP);
+    const int kk = k < NCH ? k : N - k;
+    const float2 *row = R + (a * N + b) * NCH;
+    float2 p = row[kk], q = b + 1 < N ? row[NCH + kk] : make_float2(0.0f, 0.0f);
+    if (kk == 0 || 2 * kk == N) {
+      p.y = q.y = 0.0f;
+    } else if (k >= NCH) {
+      p.y = -p.y;
+      q.y = -q.y;
+    }
+    O[i] = make_float2(p.x - q.y, p.y + q.x);
+  }
+  __syncthreads();
+  R = cube_stages<N, true, false>(O, R, tw, planes * NP, 1, [](int l) { return l * N; });
+  float *out = V + (size_t)a0 * N * N;
+  for (int i = threadIdx.x; i < planes * N * N; i += CUBE_THREADS) {
+    const int a = i / (N * N), b = (i / N) % N, c = i % N;
+    out[i] = reinterpret_cast<const float *>(R)[2 * ((a * NP + b / 2) * N + c) + (b & 1)];
+  }
+}
+
 template <int P>
 __global__ void k_gather(const float4 *__restrict__ tile_posq, const float *__restrict__ V,
                          const DBox *__restrict__ box, int na, int nb, int nc, float self_pref,
@@ -1059,9 +1309,59 @@ void twiddles(int n, std::vector<float2> &out) {
 
 size_t fft_smem(int n, int L) { return sizeof(float2) * ((size_t)n + 2 * (size_t)L * (n + 1)); }
 
+// 5-smooth sizes with compile-time transforms; other sizes take the
+// runtime-planned ones (90^3, as an example of the difference: c forward 49
+// against 16 us, a + convolution 21 against 16 us)
 #define HB_FFT_SIZES(X) \
   X(16) X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) \
-  X(80) X(96) X(128) X(160) X(192) X(256)
+  X(72) X(75) X(80) X(81) X(90) X(96) X(100) X(108) X(120) X(125) X(128) X(135) X(144) X(150) \
+  X(160) X(180) X(192) X(256)
+
+// cubes of the one-cluster transform.  One cluster is few SMs: 10.5 us at
+// 24^3 against 24.8 us in five line-pass kernels (plus the gaps between
+// them), but 23.7 against 28.6 us at 36^3 and 41 against 32 us at 48^3, where
+// an MD step gains nothing
+#define HB_CUBE_SIZES(X) X(16) X(20) X(24) X(25) X(27) X(30) X(32)
+
+bool cube_supported(int na, int nb, int nc) {
+  if (na != nb || nb != nc) return false;
+  switch (na) {
+#define HB_Q(NN) case NN:
+    HB_CUBE_SIZES(HB_Q)
+#undef HB_Q
+    return true;
+  }
+  return false;
+}
+
+// once per size, outside any stream capture
+int cube_prepare(int n) {
+  switch (n) {
+#define HB_Q(NN)                                                                                      \
+  case NN:                                                                                            \
+    HB_CUDA(cudaFuncSetAttribute(k_fft_cube<NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                 (int)cube_smem(NN)));                                                \
+    HB_CUDA(cudaFuncSetAttribute(k_fft_cube<NN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
+                                 (int)cube_smem(NN)));                                                \
+    break;
+    HB_CUBE_SIZES(HB_Q)
+#undef HB_Q
+  }
+  return HB_OK;
+}
+
+void cube_pass(int n, unsigned long long *rho, float *v, const float2 *tw, const DBox *box,
+               const float *bfac, float alpha, double *part, cudaStream_t s, bool ev) {
+  switch (n) {
+#define HB_Q(NN)                                                                                       \
+  case NN:                                                                                             \
+    if (ev) k_fft_cube<NN, true><<<CUBE_CTAS, CUBE_THREADS, cube_smem(NN), s>>>(rho, v, tw, box, bfac, alpha, part); \
+    else k_fft_cube<NN, false><<<CUBE_CTAS, CUBE_THREADS, cube_smem(NN), s>>>(rho, v, tw, box, bfac, alpha, part);   \
+    break;
+    HB_CUBE_SIZES(HB_Q)
+#undef HB_Q
+  }
+}
 
 struct SpmeLaunch {
   int na, nb, nc, nch, La, Lb, Lc;
@@ -1174,11 +1474,11 @@ void fft_passes(const SpmeLaunch &q, unsigned long long *rho, float2 *grid, floa
 
 }  // namespace
 
-// energy / virial partials written per step: one per kc plane (plane form)
-// or one per a-pass CTA (line form)
+// energy / virial partials written per step: one per CTA of the cluster (cube
+// form), per kc plane (plane form) or per a-pass CTA (line form)
 int spme_n_part(const SpmeState &S) {
   const int La = lines_per_cta(S.na);
-  return S.use_plane ? S.nch : S.nb * ((S.nch + La - 1) / La);
+  return S.use_cube ? CUBE_CTAS : S.use_plane ? S.nch : S.nb * ((S.nch + La - 1) / La);
 }
 
 int spme_set_form(hb_forcefield *ff, int param, int value) {
@@ -1189,6 +1489,9 @@ int spme_set_form(hb_forcefield *ff, int param, int value) {
     const int use = (value && plane_supported(S.na, S.nb)) ? 1 : 0;
     if (use && !S.use_plane) HB_TRY(plane_prepare(S.na));
     S.use_plane = use;
+    const int cube = (value && cube_supported(S.na, S.nb, S.nc)) ? 1 : 0;
+    if (cube && !S.use_cube) HB_TRY(cube_prepare(S.na));
+    S.use_cube = cube;
     S.n_part = spme_n_part(S);
   } else {
     S.gather_c = value;
@@ -1236,10 +1539,12 @@ int spme_setup(hb_forcefield *ff, const hb_forcefield_desc *d) {
   HB_CUDA(cudaMemcpy(S.d_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   S.use_plane = plane_supported(S.na, S.nb) ? 1 : 0;
   if (S.use_plane) HB_TRY(plane_prepare(S.na));
+  S.use_cube = cube_supported(S.na, S.nb, S.nc) ? 1 : 0;
+  if (S.use_cube) HB_TRY(cube_prepare(S.na));
   S.n_part = spme_n_part(S);
   // room for the partials of either transform form (HB_LAUNCH_FFT_PLANE)
   const int La = lines_per_cta(S.na);
-  const int max_part = std::max(S.nch, S.nb * ((S.nch + La - 1) / La));
+  const int max_part = std::max({CUBE_CTAS, S.nch, S.nb * ((S.nch + La - 1) / La)});
   HB_CUDA(cudaMalloc(&S.d_part, sizeof(double) * 2 * max_part));
   HB_CUDA(cudaMalloc(&S.d_sums, sizeof(double) * 2));
   HB_CUDA(cudaMemset(S.d_sums, 0, sizeof(double) * 2));
@@ -1280,7 +1585,10 @@ int spme_launch(hb_forcefield *ff, bool ev, cudaStream_t s) {
       default: return hb_fail(HB_ERR_INVALID_ARGUMENT, "spline order must be 4..8");
     }
   }
-  fft_passes(spme_plan(na, nb, nc), S.d_rho_fixed, S.d_grid, S.d_v, S.d_tw, sys->d_box, S.d_bfac,
+  if (S.use_cube)
+    cube_pass(na, S.d_rho_fixed, S.d_v, S.d_tw, sys->d_box, S.d_bfac, S.alpha, S.d_part, s, ev);
+  else
+    fft_passes(spme_plan(na, nb, nc), S.d_rho_fixed, S.d_grid, S.d_v, S.d_tw, sys->d_box, S.d_bfac,
              S.alpha, S.d_part, s, S.use_plane != 0, ev);
   if (n > 0) {
     switch (S.order) {
@@ -1390,7 +1698,8 @@ extern "C" int hb_spme_recip_noalloc(const float *posq, uint32_t n, const double
     return hb_fail(HB_ERR_INVALID_GRID, "SPME grid sizes must factor into 2, 3, 5, 7");
   const int nch = nc / 2 + 1;
   const int La = lines_per_cta(na), Lb = lines_per_cta(nb), Lc = lines_per_cta(nc);
-  const int n_part = nb * ((nch + La - 1) / La);
+  const bool cube = cube_supported(na, nb, nc);  // the force field's own choice
+  const int n_part = cube ? CUBE_CTAS : nb * ((nch + La - 1) / La);
   if (n_part > HB_NOALLOC_MAX_PART) return hb_fail(HB_ERR_INVALID_GRID, "grid too large");
 
   // once per device: the device address of the scratch array
@@ -1465,7 +1774,12 @@ extern "C" int hb_spme_recip_noalloc(const float *posq, uint32_t n, const double
       default: k_spread<8><<<hb_div_up(th, 256), 256, 0, s>>>(pq, dbox, na, nb, nc, rho, n); break;
     }
   }
-  fft_passes(spme_plan(na, nb, nc), rho, cgrid, v, tw, dbox, bfac, (float)alpha, part, s, false);
+  if (cube) {
+    HB_TRY(cube_prepare(na));
+    cube_pass(na, rho, v, tw, dbox, bfac, (float)alpha, part, s, true);
+  } else {
+    fft_passes(spme_plan(na, nb, nc), rho, cgrid, v, tw, dbox, bfac, (float)alpha, part, s, false);
+  }
   if (n > 0) {
     switch (order) {
       case 4: k_gather<4><<<hb_div_up(n, 128), 128, 0, s>>>(pq, v, dbox, na, nb, nc, self_pref, o, n); break;
