@@ -492,6 +492,8 @@ extern "C" int hb_forcefield_destroy(hb_forcefield *ff) {
   if (!ff) return HB_OK;
   cudaSetDevice(ff->sys->ctx->device);
   hb_context_synchronize(ff->sys->ctx);
+  for (auto &e : ff->eval_graph)
+    if (e.exec) cudaGraphExecDestroy(e.exec);
   nl_free(ff);
   bonded_free(ff);
   if (ff->spme.on) spme_free(ff);
@@ -698,6 +700,44 @@ static int force_eval(hb_forcefield *ff, bool ev, bool capturing = false) {
   return force_post(ff, ev);
 }
 
+// An evaluation outside a captured step (a program's own driver, the
+// minimiser).  The fourth of the same kind on unchanged buffers is captured,
+// and later ones replay that graph: one launch instead of the 12 to 20 and
+// the events of the eager sequence, whose issue on the host takes longer than
+// a small system's kernels.  The first ones stay eager, so that a program
+// that evaluates a few times pays for no capture.
+static int force_eval_repeated(hb_forcefield *ff, bool ev) {
+  hb_context *ctx = ff->sys->ctx;
+  hb_forcefield::EvalGraph &e = ff->eval_graph[ev ? 1 : 0];
+  if (e.gen != ff->layout_gen) {
+    if (e.exec) {
+      HB_CUDA(cudaStreamSynchronize(ctx->stream));
+      cudaGraphExecDestroy(e.exec);
+    }
+    e.exec = nullptr;
+    e.calls = 0;
+    e.gen = ff->layout_gen;
+  }
+  if (ctx->timing || g_timer || (!e.exec && ++e.calls < 4)) return force_eval(ff, ev);
+  cudaStream_t s = ctx->stream;
+  if (!e.exec) {
+    cudaGraph_t g;
+    HB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    const int rc = force_eval(ff, ev, true);
+    const cudaError_t ce = cudaStreamEndCapture(s, &g);
+    if (rc != HB_OK) return rc;
+    if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+    const cudaError_t ie = cudaGraphInstantiate(&e.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ie != cudaSuccess) {
+      e.exec = nullptr;
+      return hb_fail(HB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
+    }
+  }
+  HB_CUDA(cudaGraphLaunch(e.exec, s));
+  return HB_OK;
+}
+
 // host check of the status word: overflow is an error (the reference's
 // PackedNeighborOverflow), high water grows the buffers
 static int check_status(hb_forcefield *ff) {
@@ -722,7 +762,7 @@ extern "C" int hb_forcefield_step(hb_forcefield *ff, int level) {
   HB_REQUIRE(ff, HB_ERR_INVALID_ARGUMENT, "null force field");
   HB_REQUIRE(level == HB_FORCES_ONLY || level == HB_FORCES_AND_SCALARS, HB_ERR_INVALID_ARGUMENT,
              "bad aggregate level");
-  HB_TRY(force_eval(ff, level == HB_FORCES_AND_SCALARS));
+  HB_TRY(force_eval_repeated(ff, level == HB_FORCES_AND_SCALARS));
   return check_status(ff);
 }
 
@@ -1254,7 +1294,7 @@ extern "C" int hb_minimizer_begin(hb_minimizer *m, hb_min_report *out) {
   hb_forcefield *ff = m->ff;
   cudaStream_t s = ff->sys->ctx->stream;
   ff->sys->fix_valid = false;
-  HB_TRY(force_eval(ff, true));
+  HB_TRY(force_eval_repeated(ff, true));
   HB_TRY(min_init(m, s));
   HB_CUDA(cudaMemcpyAsync(out, m->d_rep, sizeof(hb_min_report), cudaMemcpyDeviceToHost, s));
   HB_CUDA(cudaStreamSynchronize(s));
@@ -1280,7 +1320,7 @@ extern "C" int hb_minimizer_iterate(hb_minimizer *m, uint32_t n, hb_min_report *
     for (uint32_t k = 0; k < chunk; ++k) {
       HB_TRY(min_trial(m, s));
       if (m->cons) HB_TRY(cons_project(m->cons, &m->d_st->skip, s));
-      HB_TRY(force_eval(ff, true));
+      HB_TRY(force_eval_repeated(ff, true));
       HB_TRY(min_finish(m, k, s));
     }
     HB_CUDA(cudaMemcpyAsync(&after, m->d_st, sizeof(MinState), cudaMemcpyDeviceToHost, s));

@@ -327,6 +327,12 @@ uint64_t hb_next_uid();
 struct hb_forcefield {
   hb_system *sys = nullptr;
   uint64_t uid = hb_next_uid();
+  // graphs of repeated evaluations: without and with energies
+  struct EvalGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t gen = 0;    // layout_gen it was captured at
+    uint32_t calls = 0;  // eager calls since that changed
+  } eval_graph[2];
   // ---- parameters
   int lj_on = 0, coul_on = 0;
   uint32_t n_types = 0;
