@@ -605,8 +605,7 @@ extern "C" int hb_forcefield_create(hb_system *sys, const hb_forcefield_desc *d,
   hb_forcefield *ff = new hb_forcefield();
   *ff = tmp;
   ff->sys = sys;
-  // pair kernel: the balanced queue form (with or without energies); exact
-  // pairs take the compacted form with per-pair fixed point and minimum image
+  // exact pairs: per-pair fixed point and minimum image
   ff->exact_pairs = d->pair_mode == HB_PAIRS_EXACT;
   HB_CUDA(cudaSetDevice(sys->ctx->device));
   HB_CUDA(cudaMalloc(&ff->d_lj, sizeof(float4) * ff->h_lj.size()));

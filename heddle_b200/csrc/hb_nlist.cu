@@ -17,8 +17,8 @@
 //     mask per j-atom (bit m: the pair with i-atom m is in the exclusion
 //     list), so the pair kernel never scans exclusion lists for ordinary
 //     pairs;
-//   * the self tile is entry 0 of each i-tile and is evaluated with a half
-//     rotation (each unordered pair once);
+//   * the self tile is entry 0 of each i-tile (the pair kernel takes each of
+//     its unordered pairs once);
 //   * entries live in a fixed-size slab per i-tile (sized from a counting
 //     pass at the first build), so a rebuild is one pass and the layout is
 //     identical run to run;

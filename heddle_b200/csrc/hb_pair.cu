@@ -800,7 +800,7 @@ int pair_launch(hb_forcefield *ff, bool ev, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------
-// Multi-system pair launch (replica batches): one persistent k_pair4 over
+// Multi-system pair launch (replica batches): one persistent k_pair over
 // the work items of every member, each item finding its member by a binary
 // search of the members' first items.  Members must share the pair physics
 // (types, tables, cut-offs, Ewald alpha, switch) and take the force-only,

@@ -33,7 +33,8 @@
 // the c pass writes kc-major planes instead, and one whole-plane pass per
 // kc replaces fft_b, fft_a and ifft_b: both forward transforms, the
 // influence function and both inverse transforms run in place on the plane
-// in shared memory (radix-16 and radix-8 stages).  Deterministic by
+// in shared memory (radix-16 and radix-8 stages).  Cubes up to 32^3 take one
+// kernel of one cluster for all of it (k_fft_cube).  Deterministic by
 // construction.
 #include <cooperative_groups.h>
 
