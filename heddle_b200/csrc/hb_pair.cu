@@ -96,7 +96,8 @@ __device__ __forceinline__ void red_add(unsigned long long *p, long long v) {
 // entry.  A pair force component above 0.06 hartree/bohr takes the int64
 // path instead, so the int32 sums cannot wrap (32 x 0.06 x 2^30 < 2^31).
 // With EV the energy and virial halves of each pair are int32 sums at 2^28
-// (guard 0.25 hartree), and the LJ energy total is summed per lane in int64.
+// (guard 0.24 hartree: 32 x 0.24 x 2^28 < 2^31, where 0.25 would wrap), and
+// the LJ energy total is summed per lane in int64.
 //
 // EXACT: every pair force is converted to int64 (2^40) by itself and takes
 // the minimum image of the two stored positions, so it is a function of the
@@ -120,7 +121,10 @@ __device__ __forceinline__ void red_add(unsigned long long *p, long long v) {
 #define PK_FMAX 0.06f
 #define PK_ESHIFT 12              // 2^40 / 2^28
 #define PK_ESCALE 268435456.0f    // 2^28
-#define PK_EMAX 0.25f
+#define PK_EMAX 0.24f
+// 32 terms at the guards, each rounded to an integer, fit an int32
+static_assert(32.0 * (PK_FMAX * (double)PK_SCALE + 0.5) < 2147483648.0, "force sums may wrap");
+static_assert(32.0 * (PK_EMAX * (double)PK_ESCALE + 0.5) < 2147483648.0, "energy sums may wrap");
 
 template <bool EV, bool SCALED, bool EXACT>
 struct PairWarp {

@@ -94,3 +94,34 @@ def test_forces_match_oracle(ctx, form, edge, tilt, n, n_types, scaled):
     assert off(sys_.forces(), Fo) <= 1.0
     ff.close()
     sys_.close()
+
+
+def test_sums_at_the_guard_do_not_wrap(ctx):
+    """32 atoms at one point and one atom 4 bohr from them, at the minimum's
+    side of sigma = r, where a pair's virial is 24 eps exactly: with eps at and
+    around 1 / 48 each of the 32 pairs gives the single atom a half of 0.25
+    hartree, 2^26 units, and 32 of those are 2^31."""
+    n, L = 33, U.angstrom_au(13.6)
+    rc = U.angstrom_au(6.0)
+    pos = np.zeros((n, 3))
+    pos[32, 0] = 4.0
+    types = np.zeros(n, dtype=np.uint32)
+    types[32] = 1
+    for k in range(-4, 5):
+        eps = np.zeros((2, 2))
+        eps[0, 1] = eps[1, 0] = (0.5 + k * 2.0 ** -25) / 24.0
+        spec = S.SystemSpec(
+            name="guard", positions=pos, velocities=np.zeros((n, 3)), masses=np.full(n, 1.0e4),
+            charges=np.zeros(n), types=types, box=np.array([L, L, L, 0.0, 0.0, 0.0]), n_types=2,
+            lj_sigma=np.full((2, 2), 4.0), lj_epsilon=eps, lj_cutoff=np.full((2, 2), rc),
+            lj_switch=np.full((2, 2), rc), alpha=None, r_cut_coul=None, grid=None, excl_offsets=None,
+            excl_partners=None, excl_lj=None, excl_coul=None, r_skin=U.angstrom_au(0.6))
+        sys_ = hb.System.from_spec(ctx, spec)
+        ff = hb.ForceField.from_spec(sys_, spec)
+        ff.step(scalars=True)
+        _, w = ff.per_atom()
+        ff.close()
+        sys_.close()
+        # 2^-28 units; rsqrt's 2^-22 in sr^12 makes 3e-6 of 0.25 at most
+        assert np.abs(w[:32] - 0.25).max() <= 5e-6, (k, w[:32])
+        assert abs(w[32] - 8.0) <= 32 * 5e-6, (k, w[32])
