@@ -517,7 +517,7 @@ extern "C" int hb_forcefield_create(hb_system *sys, const hb_forcefield_desc *d,
   hb_forcefield tmp;
   double rc_max = 0.0;
   if (d->lj_enabled) {
-    HB_REQUIRE(d->n_types >= 1 && d->n_types <= 64, HB_ERR_INVALID_ARGUMENT,
+    HB_REQUIRE(d->n_types >= 1 && d->n_types <= HB_MAX_TYPES, HB_ERR_INVALID_ARGUMENT,
                "LJ needs 1..64 particle types");
     HB_REQUIRE(d->lj_sigma && d->lj_epsilon && d->lj_cutoff && d->lj_switch,
                HB_ERR_INVALID_ARGUMENT, "LJ tables are required");

@@ -52,6 +52,7 @@ int hb_fail(int code, const std::string &msg);
 #define HB_VFIX_SCALE 72057594037927936.0   /* 2^56 per bohr / aut */
 
 #define HB_TILE 32
+#define HB_MAX_TYPES 64             /* particle types of a Lennard-Jones table */
 #define HB_SENTINEL 0xFFFFFFFFu
 
 // status word bits (kernels/neighbor.cu:634-669 layout, plus build bits)

@@ -710,12 +710,18 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PAIR_MIN_BLOCKS(EV, EXACT, MULT
   }
 }
 
-// The type tables of more than about 30 types do not fit beside the warps'
-// shared memory within the default 48 KB
+// dynamic shared memory: the type tables
+constexpr size_t table_bytes(size_t n_types) { return (sizeof(float4) + sizeof(float)) * n_types * n_types; }
+
+// Tables of more than 28 types may not fit beside the warps' shared memory
+// within the default 48 KB.  The limit is a property of the kernel in the
+// whole process, so it is only ever set to the largest table's size: another
+// thread's launch with a smaller table leaves it where it is.
 template <class K>
 int allow_smem(K kernel, size_t dynamic) {
   if (dynamic > 16u * 1024u)
-    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic));
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)table_bytes(HB_MAX_TYPES)));
   return HB_OK;
 }
 
@@ -746,7 +752,7 @@ uint32_t pair_blocks_of(const hb_forcefield *ff, bool wide) {
 
 template <bool EV, bool SCALED, bool SWITCH, bool EXACT>
 int launch_t(hb_forcefield *ff, cudaStream_t s, const PairParams &P) {
-  size_t smem = (sizeof(float4) + sizeof(float)) * (size_t)P.n_types * P.n_types;
+  const size_t smem = table_bytes((size_t)P.n_types);
   const uint32_t chunk = pair_chunk_of(ff);  // entries per work item
   const uint32_t chunks = hb_div_up(P.slab, chunk);
   const uint32_t items = P.n_tiles * chunks;
@@ -872,7 +878,7 @@ int pair_launch_batch(hb_forcefield *const *ffs, uint32_t n, const void *d_table
   P.alpha = a->alpha;
   P.c2a = 2.0f * a->alpha / 1.7724538509055160273f;
   P.nl2e = -1.44269504088896340736f;
-  size_t smem = (sizeof(float4) + sizeof(float)) * (size_t)P.n_types * P.n_types;
+  const size_t smem = table_bytes((size_t)P.n_types);
   const uint32_t grid = std::min<uint32_t>(
       (uint32_t)a->sys->ctx->n_sm * pair_blocks_of(a, true), hb_div_up(items_total, PK_WARPS));
   HB_CUDA(cudaMemsetAsync(d_work, 0, sizeof(uint32_t), s));

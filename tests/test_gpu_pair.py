@@ -5,6 +5,8 @@ orthorhombic and tilted minimum images, one and several atom types (more than
 with and without energies, the exact form, and any split of the entries into
 work items."""
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -125,3 +127,40 @@ def test_sums_at_the_guard_do_not_wrap(ctx):
         # 2^-28 units; rsqrt's 2^-22 in sr^12 makes 3e-6 of 0.25 at most
         assert np.abs(w[:32] - 0.25).max() <= 5e-6, (k, w[:32])
         assert abs(w[32] - 8.0) <= 32 * 5e-6, (k, w[32])
+
+
+def test_two_threads_with_tables_of_different_sizes(ctx):
+    """Type tables of more than 28 types need more shared memory than a kernel
+    has by default, and that limit belongs to the process: two contexts in two
+    threads, one with the largest table and one with a smaller, evaluate at
+    the same time without lowering it under each other."""
+    specs = [system(97, 13.6, (0.0, 0.0, 0.0), t, False) for t in (64, 40)]
+    want, errors = [], []
+    for spec in specs:
+        sys_ = hb.System.from_spec(ctx, spec)
+        ff = hb.ForceField.from_spec(sys_, spec)
+        ff.step()
+        want.append(sys_.forces())
+        ff.close()
+        sys_.close()
+
+    def work(k):
+        try:
+            own = hb.Context(0)
+            own.timing(True)  # every evaluation launches its kernels one by one
+            sys_ = hb.System.from_spec(own, specs[k])
+            ff = hb.ForceField.from_spec(sys_, specs[k])
+            for _ in range(1000):
+                ff.step()
+            assert np.array_equal(sys_.forces(), want[k])
+            for o in (ff, sys_, own):
+                o.close()
+        except Exception as e:
+            errors.append((k, e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
