@@ -1059,6 +1059,21 @@ int nl_rebuild(hb_forcefield *ff, bool gated, cudaStream_t s) {
   return nl_launch(ff, gate, s, true, false, true);
 }
 
+// The dynamic shared-memory limit of a kernel belongs to the process: it is
+// set to what the device has, not to this list's candidate capacity, which a
+// force field with more candidates would then be refused.
+template <class K>
+static int allow_largest_smem(K kernel) {
+  int device = 0, largest = 0;
+  cudaFuncAttributes a;
+  HB_CUDA(cudaGetDevice(&device));
+  HB_CUDA(cudaDeviceGetAttribute(&largest, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  HB_CUDA(cudaFuncGetAttributes(&a, kernel));
+  HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               largest - (int)a.sharedSizeBytes));
+  return HB_OK;
+}
+
 // First build: counting pass, slab size = 1.5 x the largest tile count + 4,
 // then the fill pass.  Host-synchronous; runs at force-field creation and
 // when the host grows the slabs after a high-water signal.
@@ -1081,10 +1096,8 @@ int nl_first_build(hb_forcefield *ff) {
     if (mc <= ff->maxc && ff->maxc >= want_c) break;
     ff->maxc = std::max(want_c, ff->maxc);
     ff->layout_gen++;
-    HB_CUDA(cudaFuncSetAttribute(k_nl_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(uint32_t) * (3u * ff->maxc + 1u))));
-    HB_CUDA(cudaFuncSetAttribute(k_nl_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(uint32_t) * (3u * ff->maxc + 1u))));
+    HB_TRY(allow_largest_smem(k_nl_tile<false>));
+    HB_TRY(allow_largest_smem(k_nl_tile<true>));
   }
   std::vector<uint32_t> nent(ff->n_tiles);
   HB_CUDA(cudaMemcpyAsync(nent.data(), ff->d_tile_nent, sizeof(uint32_t) * ff->n_tiles,

@@ -53,3 +53,19 @@ def test_pair_set_matches_oracle(ctx, case):
     sys_.close()
     assert dup == 0
     assert np.array_equal(pairs, ref)
+
+
+def test_candidate_capacities_of_two_force_fields(ctx):
+    """Cut-offs that reach more than 640 tiles take more shared memory in the
+    tile build than its first size: a second force field with fewer
+    candidates leaves the first one's rebuild as it was."""
+    specs = [S.spc_water(30000, r_cut_A=40.0, skin_A=4.0, seed=1),
+             S.spc_water(20000, r_cut_A=36.0, skin_A=3.6, seed=1)]
+    systems = [hb.System.from_spec(ctx, spec) for spec in specs]
+    ffs = [hb.ForceField.from_spec(s, spec, reciprocal=False) for s, spec in zip(systems, specs)]
+    entries = [ff.stats()["entries"] for ff in ffs]
+    for ff, e in zip(ffs, entries):
+        assert ff.pre_step(force=True)
+        assert ff.stats()["entries"] == e
+    for o in ffs + systems:
+        o.close()
