@@ -376,8 +376,8 @@ class ForceField:
                    pair_chunk: int | None = None, fft_plane: bool | None = None,
                    gather_per_offset: bool | None = None, pair_quota: int | None = None) -> None:
         """Launch shapes (autotuned): resident blocks per SM of the persistent
-        pair kernel, its packed entries per work item and work items per
-        warp (0: persistent blocks); the whole-plane
+        pair kernel (0: by form), its packed entries per work item (0: by
+        size) and work items per warp (0: persistent blocks); the whole-plane
         transform pass (where the grid has one) or line passes; the gather
         with one thread per (atom, c offset) or per atom.  nl_slab rebuilds
         the packed list at once into slabs of that many entries per i-tile

@@ -785,7 +785,8 @@ extern "C" int hb_forcefield_pre_step(hb_forcefield *ff, int force, int *rebuilt
 extern "C" int hb_forcefield_set_launch(hb_forcefield *ff, int param, int value) {
   HB_REQUIRE(ff, HB_ERR_INVALID_ARGUMENT, "null force field");
   if (param == HB_LAUNCH_PAIR_BLOCKS_PER_SM) {
-    HB_REQUIRE(value >= 1 && value <= 8, HB_ERR_INVALID_ARGUMENT, "pair blocks per SM in 1..8");
+    HB_REQUIRE(value >= 0 && value <= 8, HB_ERR_INVALID_ARGUMENT,
+               "pair blocks per SM in 1..8 (0: by form)");
     ff->pair_blocks_per_sm = value;
   } else if (param == HB_LAUNCH_NL_SLAB) {
     HB_REQUIRE(value >= 2, HB_ERR_INVALID_ARGUMENT, "neighbour slab must hold at least 2 entries");
@@ -799,7 +800,8 @@ extern "C" int hb_forcefield_set_launch(hb_forcefield *ff, int param, int value)
     HB_REQUIRE(value >= 0 && value <= 4096, HB_ERR_INVALID_ARGUMENT, "pair work quota in 0..4096");
     ff->pair_quota = value;
   } else if (param == HB_LAUNCH_PAIR_CHUNK) {
-    HB_REQUIRE(value >= 1 && value <= 64, HB_ERR_INVALID_ARGUMENT, "pair entry chunk in 1..64");
+    HB_REQUIRE(value >= 0 && value <= 64, HB_ERR_INVALID_ARGUMENT,
+               "pair entry chunk in 1..64 (0: by size)");
     ff->pair_chunk = value;
   } else if (param == HB_LAUNCH_FFT_PLANE || param == HB_LAUNCH_GATHER_FORM) {
     HB_TRY(spme_set_form(ff, param, value));

@@ -55,9 +55,9 @@ enum {
 /* launch-shape parameters of hb_forcefield_set_launch (autotuned) */
 enum {
   HB_LAUNCH_PAIR_BLOCKS_PER_SM = 0, /* resident blocks of the persistent pair kernel
-                                       per SM (1..8; by default as many as fit,
-                                       fewer with a reciprocal part, whose
-                                       concurrent chain needs the room) */
+                                       per SM (1..8); 0 (default) by form: as many
+                                       as fit, fewer with a reciprocal part, whose
+                                       concurrent chain needs the room */
   HB_LAUNCH_NL_SLAB = 1,            /* packed entries per i-tile slab (>= 2): the
                                        list is rebuilt at once into slabs of this
                                        size; more than 3/4 full grows them again
@@ -67,10 +67,10 @@ enum {
                                        halts the force field until a larger slab
                                        is set */
   HB_LAUNCH_PAIR_CHUNK = 2,         /* packed entries per work item of the
-                                       persistent pair kernel (1..64; by default 1
-                                       to 4 by system size):
-                                       shorter items balance better, longer ones
-                                       reload the i-tile less often */
+                                       persistent pair kernel (1..64); 0 (default)
+                                       1 to 4 by system size: shorter items balance
+                                       better, longer ones reload the i-tile less
+                                       often */
   HB_LAUNCH_FFT_PLANE = 3,          /* 1 (default where supported: 64 x 64 and
                                        128 x 128 (a, b) planes): whole-plane FFT
                                        pass, and the one-cluster transform of

@@ -12,6 +12,7 @@ import pytest
 
 import heddle_b200 as hb
 import oracle as O
+from heddle_b200 import HeddleError
 from heddle_b200 import systems as S
 from heddle_b200 import units as U
 
@@ -164,3 +165,24 @@ def test_two_threads_with_tables_of_different_sizes(ctx):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_launch_defaults_can_be_restored(ctx):
+    """0 gives the pair kernel's work item and residency back to the rules by
+    size and form; values that are out of range stay refused."""
+    spec = system(161, 13.6, (0.0, 0.0, 0.0), 3, False)
+    sys_ = hb.System.from_spec(ctx, spec)
+    ff = hb.ForceField.from_spec(sys_, spec)
+    ff.step()
+    F = sys_.forces()
+    for kw in (dict(pair_chunk=16), dict(pair_blocks_per_sm=3), dict(pair_chunk=0),
+               dict(pair_blocks_per_sm=0)):
+        ff.set_launch(**kw)
+        ff.step()
+        assert np.array_equal(sys_.forces(), F), kw
+    for kw in (dict(pair_chunk=-1), dict(pair_chunk=65), dict(pair_blocks_per_sm=-1),
+               dict(pair_blocks_per_sm=9)):
+        with pytest.raises(HeddleError):
+            ff.set_launch(**kw)
+    ff.close()
+    sys_.close()
