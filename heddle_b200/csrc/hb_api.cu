@@ -699,6 +699,24 @@ static int force_eval(hb_forcefield *ff, bool ev, bool capturing = false) {
   return force_post(ff, ev);
 }
 
+// The end of a capture whose calls returned rc: an executable graph, or the
+// first error.  The captured graph is given back in every case.
+static int end_capture(cudaStream_t s, int rc, cudaGraphExec_t *exec, const char *what) {
+  cudaGraph_t g = nullptr;
+  const cudaError_t ce = cudaStreamEndCapture(s, &g);
+  if (rc == HB_OK && ce != cudaSuccess)
+    rc = hb_fail(HB_ERR_CUDA, std::string(what) + " capture: " + cudaGetErrorString(ce));
+  if (rc == HB_OK) {
+    const cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
+    if (ie != cudaSuccess) {
+      *exec = nullptr;
+      rc = hb_fail(HB_ERR_CUDA, std::string(what) + " instantiate: " + cudaGetErrorString(ie));
+    }
+  }
+  if (g) cudaGraphDestroy(g);
+  return rc;
+}
+
 // An evaluation outside a captured step (a program's own driver, the
 // minimiser).  The fourth of the same kind on unchanged buffers is captured,
 // and later ones replay that graph: one launch instead of the 12 to 20 and
@@ -720,17 +738,14 @@ static int force_eval_repeated(hb_forcefield *ff, bool ev) {
   if (ctx->timing || g_timer || (!e.exec && ++e.calls < 4)) return force_eval(ff, ev);
   cudaStream_t s = ctx->stream;
   if (!e.exec) {
-    cudaGraph_t g;
     HB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const int rc = force_eval(ff, ev, true);
-    const cudaError_t ce = cudaStreamEndCapture(s, &g);
-    if (rc != HB_OK) return rc;
-    if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-    const cudaError_t ie = cudaGraphInstantiate(&e.exec, g, 0);
-    cudaGraphDestroy(g);
-    if (ie != cudaSuccess) {
-      e.exec = nullptr;
-      return hb_fail(HB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
+    const int rc = end_capture(s, force_eval(ff, ev, true), &e.exec, "graph");
+    if (rc != HB_OK) {
+      // nothing of the capture ran: what cannot be made a graph (no memory
+      // for one, say) is still evaluated as it was before
+      cudaGetLastError();
+      e.calls = 0;
+      return force_eval(ff, ev);
     }
   }
   HB_CUDA(cudaGraphLaunch(e.exec, s));
@@ -1415,19 +1430,12 @@ extern "C" int hb_integrator_step(hb_integrator *it, hb_forcefield *ff, hb_const
 static int capture_step(hb_integrator *it, hb_forcefield *ff, hb_constraints *cons, bool move,
                         cudaGraphExec_t *exec) {
   cudaStream_t s = it->sys->ctx->stream;
-  cudaGraph_t g;
   HB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   const uint64_t step = it->step;
   int rc = one_step(it, ff, cons, move, true);
   if (rc == HB_OK && move) rc = baro_move(it->baro, ff, true);
   it->step = step;
-  cudaError_t ce = cudaStreamEndCapture(s, &g);
-  if (rc != HB_OK) return rc;
-  if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-  cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  if (ie != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
-  return HB_OK;
+  return end_capture(s, rc, exec, "graph");
 }
 
 static void drop_exchange_graphs(hb_integrator *it) {
@@ -1572,18 +1580,11 @@ static int exchange_step(hb_integrator *it, hb_forcefield *ff, hb_constraints *c
 static int capture_exchange(hb_integrator *it, hb_forcefield *ff, hb_constraints *cons, bool move,
                             const ExchangeOut &xo, cudaGraphExec_t *exec) {
   cudaStream_t s = it->sys->ctx->stream;
-  cudaGraph_t g;
   HB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   const uint64_t step = it->step;
   int rc = exchange_step(it, ff, cons, move, true, xo);
   it->step = step;
-  cudaError_t ce = cudaStreamEndCapture(s, &g);
-  if (rc != HB_OK) return rc;
-  if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-  cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  if (ie != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
-  return HB_OK;
+  return end_capture(s, rc, exec, "graph");
 }
 
 static bool page_locked(const void *p) {
@@ -1671,18 +1672,18 @@ static int count_kernel_nodes(cudaGraph_t g, uint64_t &kernels) {
 static int count_captured(hb_integrator *it, hb_forcefield *ff, hb_constraints *cons, bool step,
                           bool move, uint64_t &kernels) {
   cudaStream_t s = it->sys->ctx->stream;
-  cudaGraph_t g;
+  cudaGraph_t g = nullptr;
   HB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   const uint64_t st = it->step;
   int rc = step ? one_step(it, ff, cons, false, false) : HB_OK;
   if (rc == HB_OK && move) rc = baro_move(it->baro, ff, false);
   it->step = st;
   cudaError_t ce = cudaStreamEndCapture(s, &g);
-  if (rc != HB_OK) return rc;
-  if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
+  if (rc == HB_OK && ce != cudaSuccess)
+    rc = hb_fail(HB_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
   kernels = 0;
-  rc = count_kernel_nodes(g, kernels);
-  cudaGraphDestroy(g);
+  if (rc == HB_OK) rc = count_kernel_nodes(g, kernels);
+  if (g) cudaGraphDestroy(g);
   return rc;
 }
 
@@ -1817,7 +1818,6 @@ static int batch_capture(hb_batch *b) {
   b->multi = batch_multi_ok(b);
   if (b->multi) HB_TRY(pair_batch_table(b->ffs.data(), (uint32_t)n, b->d_members, &b->items));
   cudaStream_t m = b->ctx->stream;
-  cudaGraph_t g;
   HB_CUDA(cudaStreamBeginCapture(m, cudaStreamCaptureModeThreadLocal));
   int rc = cudaEventRecord(b->fork, m) == cudaSuccess ? HB_OK : HB_ERR_CUDA;
   std::vector<uint64_t> steps(n);
@@ -1862,13 +1862,7 @@ static int batch_capture(hb_batch *b) {
         rc = hb_fail(HB_ERR_CUDA, "batch join");
     }
   }
-  cudaError_t ce = cudaStreamEndCapture(m, &g);
-  if (rc != HB_OK) return rc;
-  if (ce != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("batch capture: ") + cudaGetErrorString(ce));
-  cudaError_t ie = cudaGraphInstantiate(&b->exec, g, 0);
-  cudaGraphDestroy(g);
-  if (ie != cudaSuccess) return hb_fail(HB_ERR_CUDA, std::string("batch instantiate: ") + cudaGetErrorString(ie));
-  return HB_OK;
+  return end_capture(m, rc, &b->exec, "batch");
 }
 
 extern "C" int hb_batch_set_pair_form(hb_batch *b, int one_launch) {
