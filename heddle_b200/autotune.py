@@ -13,8 +13,11 @@ residency, its entries per work item (shorter items balance better, longer
 ones reload the i-tile less often), the reciprocal transform form (the
 whole-plane pass or line passes, where both exist) and the gather form
 (one thread per (atom, c offset) or per atom, spline orders 4 and 8).
-Results are keyed by a size class (atoms, grid) and can be kept in a JSON
-cache file.
+The pair kernel's own rules (0: residency by form, items by size) take part
+in both sweeps and stay unless a fixed value is faster by more than MARGIN:
+a fixed residency also holds for evaluations with energies, which the timed
+steps may not contain.  Results are keyed by the pair kernel they were timed
+with and a size class (atoms, grid) and can be kept in a JSON cache file.
 """
 
 from __future__ import annotations
@@ -27,9 +30,18 @@ from . import _native as N
 from .api import Constraints, ForceField, Integrator, System
 
 
+# the pair kernel that cached results belong to: changed with the kernel, so
+# that values tuned for another one are not taken over
+PAIR_KERNEL = "k_pair"
+
+# a fixed launch shape replaces the rule only when it is this much faster
+# (runs of one shape differ by 1 to 2 %)
+MARGIN = 0.02
+
+
 def size_class(spec) -> str:
     grid = "x".join(str(g) for g in spec.grid) if spec.grid else "none"
-    return f"n{spec.n}-grid{grid}-rc{spec.r_cut_coul or 0:.3f}"
+    return f"{PAIR_KERNEL}-n{spec.n}-grid{grid}-rc{spec.r_cut_coul or 0:.3f}"
 
 
 def _time_steps(ctx, sys_, ff, cons, integrator_kwargs, steps, warm) -> float:
@@ -44,8 +56,8 @@ def _time_steps(ctx, sys_, ff, cons, integrator_kwargs, steps, warm) -> float:
 
 
 def tune_skin(ctx, sys_: System, spec, cons: Constraints | None, integrator_kwargs: dict,
-              candidates_A=(1.2, 1.6, 2.0, 2.5, 3.0), residencies=(4, 5, 6, 7, 8),
-              chunks=(2, 4, 8, 16), steps: int = 150, warm: int = 20,
+              candidates_A=(1.2, 1.6, 2.0, 2.5, 3.0), residencies=(0, 3, 4, 5, 6),
+              chunks=(0, 1, 2, 4, 8), steps: int = 150, warm: int = 20,
               cache: Path | None = None) -> dict:
     """Time `steps` graph-mode MD steps per candidate skin (angstrom), then
     per launch-shape knob at the best skin; return {"best_A": skin,
@@ -72,12 +84,14 @@ def tune_skin(ctx, sys_: System, spec, cons: Constraints | None, integrator_kwar
     best = min(times, key=times.get)
     ff = ForceField.from_spec(sys_, spec, r_skin=U.angstrom_au(best))
 
-    def sweep(param, values):
+    def sweep(param, values, zero_is_rule=True):
         t = {}
         for v in values:
             N.check(ff.lib.hb_forcefield_set_launch(ff.h, param, int(v)))
             t[v] = _time_steps(ctx, sys_, ff, cons, integrator_kwargs, steps, warm)
         b = min(t, key=t.get)
+        if zero_is_rule and 0 in t and t[b] > (1.0 - MARGIN) * t[0]:
+            b = 0
         N.check(ff.lib.hb_forcefield_set_launch(ff.h, param, int(b)))
         return b, {str(k): v for k, v in t.items()}
 
@@ -89,9 +103,9 @@ def tune_skin(ctx, sys_: System, spec, cons: Constraints | None, integrator_kwar
     grid = spec.grid if spec.alpha is not None else None
     if grid is not None:
         if grid[0] == grid[1] and grid[0] in (64, 128):
-            result["fft_plane"], result["fft_plane_ms"] = sweep(N.HB_LAUNCH_FFT_PLANE, (1, 0))
+            result["fft_plane"], result["fft_plane_ms"] = sweep(N.HB_LAUNCH_FFT_PLANE, (1, 0), False)
         if spec.order in (4, 8):
-            result["gather_form"], result["gather_form_ms"] = sweep(N.HB_LAUNCH_GATHER_FORM, (1, 0))
+            result["gather_form"], result["gather_form_ms"] = sweep(N.HB_LAUNCH_GATHER_FORM, (1, 0), False)
     ff.close()
     if cache is not None:
         data = json.loads(cache.read_text()) if cache.exists() else {}
