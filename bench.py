@@ -72,6 +72,24 @@ def parse():
     return p.parse_args()
 
 
+PAIR_KERNEL = "k_pair<0,0,1,0,0>"  # the force-only form of the water boxes
+
+
+def pair_traffic(molecules, skin_A, path=ROOT / "profiles" / "pair_kernel_traffic.json"):
+    """Measured DRAM bytes per launch of the present pair kernel at this box
+    and skin, or None where no capture of exactly that is kept."""
+    try:
+        record = json.loads(path.read_text())
+        if record["kernel"] != PAIR_KERNEL:
+            return None
+        for run in record["captures"]:
+            if run["molecules"] == molecules and abs(run["skin_A"] - skin_A) < 1e-6:
+                return run["dram_bytes_per_launch"]
+    except (OSError, ValueError, KeyError, TypeError):
+        pass
+    return None
+
+
 def workload_config(args, spec, world):
     return {
         "workload": f"spc-water-{args.molecules} (N={spec.n} atoms), SETTLE, LJ+erfc r_cut 9 A, "
@@ -443,13 +461,7 @@ def run_ours(args):
 
     line = None
     if rank == 0:
-        traffic = None
-        tf = ROOT / "profiles" / "pair_kernel_traffic.json"
-        if tf.exists():
-            try:
-                traffic = json.loads(tf.read_text()).get("dram_bytes_per_launch_full_size")
-            except Exception:
-                traffic = None
+        traffic = pair_traffic(args.molecules, args.skin)
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": max(3, args.warmup) + args.equilibrate, "ms_per_step": t_ms / args.steps, "higher_is_better": True,
@@ -471,7 +483,8 @@ def run_ours(args):
                          "peak_source": peak_kind,
                          "note": "algorithmic bytes 28 B/atom per launch; the kernel is latency- and "
                                  "issue-limited (no pipe saturated), not HBM-bound; traffic is the "
-                                 "packed neighbour entries read once per launch"},
+                                 "DRAM bytes of one launch of this kernel at this box and skin, "
+                                 "captured before, null where that was not captured"},
             "step_roofline": {"bytes_per_step": step_bytes,
                               "achieved_gbs": step_bytes / (t_ms / args.steps * 1e-3) / 1e9,
                               "frac": step_bytes / (t_ms / args.steps * 1e-3) / 1e9 / peak},
