@@ -850,8 +850,11 @@ __global__ void __launch_bounds__(PLANE_THREADS) k_fft_plane(
 // shared memory (along a: forward, influence function, inverse), then its
 // slab again.  Bound: latency -- each stage is one or two butterflies per
 // thread and a barrier; what it saves is five kernels' launches, tails and
-// global round trips.  256 threads and at most 64 registers, so that its
-// CTAs fit beside resident pair blocks.
+// global round trips.  384 threads of 56 to 79 registers, 5 to 34 KB of
+// shared memory.  A cell of these grids has fewer pair work items than the
+// pair kernel may keep resident, so its CTAs find room whatever that
+// residency is (343 waters: 890, 896, 887, 894, 900 us per 20 steps at 2 to 6
+// blocks per SM).
 // ---------------------------------------------------------------------
 constexpr int CUBE_CTAS = 8, CUBE_THREADS = 384;
 
@@ -1310,8 +1313,8 @@ void twiddles(int n, std::vector<float2> &out) {
 
 size_t fft_smem(int n, int L) { return sizeof(float2) * ((size_t)n + 2 * (size_t)L * (n + 1)); }
 
-// 5-smooth sizes with compile-time transforms; other sizes take the
-// runtime-planned ones (90^3, as an example of the difference: c forward 49
+// sizes with compile-time transforms: the 5-smooth ones from 16 to 192 but 18
+// and 162, and 256; other sizes take the runtime-planned ones (90^3, as an example of the difference: c forward 49
 // against 16 us, a + convolution 21 against 16 us)
 #define HB_FFT_SIZES(X) \
   X(16) X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) \
@@ -1335,21 +1338,8 @@ bool cube_supported(int na, int nb, int nc) {
   return false;
 }
 
-// once per size, outside any stream capture
-int cube_prepare(int n) {
-  switch (n) {
-#define HB_Q(NN)                                                                                      \
-  case NN:                                                                                            \
-    HB_CUDA(cudaFuncSetAttribute(k_fft_cube<NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                 (int)cube_smem(NN)));                                                \
-    HB_CUDA(cudaFuncSetAttribute(k_fft_cube<NN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                 (int)cube_smem(NN)));                                                \
-    break;
-    HB_CUBE_SIZES(HB_Q)
-#undef HB_Q
-  }
-  return HB_OK;
-}
+// within the default limit of dynamic shared memory (beside 192 B of static)
+static_assert(cube_smem(32) <= 47 * 1024, "the cube transform needs a raised limit");
 
 void cube_pass(int n, unsigned long long *rho, float *v, const float2 *tw, const DBox *box,
                const float *bfac, float alpha, double *part, cudaStream_t s, bool ev) {
@@ -1490,9 +1480,7 @@ int spme_set_form(hb_forcefield *ff, int param, int value) {
     const int use = (value && plane_supported(S.na, S.nb)) ? 1 : 0;
     if (use && !S.use_plane) HB_TRY(plane_prepare(S.na));
     S.use_plane = use;
-    const int cube = (value && cube_supported(S.na, S.nb, S.nc)) ? 1 : 0;
-    if (cube && !S.use_cube) HB_TRY(cube_prepare(S.na));
-    S.use_cube = cube;
+    S.use_cube = (value && cube_supported(S.na, S.nb, S.nc)) ? 1 : 0;
     S.n_part = spme_n_part(S);
   } else {
     S.gather_c = value;
@@ -1541,7 +1529,6 @@ int spme_setup(hb_forcefield *ff, const hb_forcefield_desc *d) {
   S.use_plane = plane_supported(S.na, S.nb) ? 1 : 0;
   if (S.use_plane) HB_TRY(plane_prepare(S.na));
   S.use_cube = cube_supported(S.na, S.nb, S.nc) ? 1 : 0;
-  if (S.use_cube) HB_TRY(cube_prepare(S.na));
   S.n_part = spme_n_part(S);
   // room for the partials of either transform form (HB_LAUNCH_FFT_PLANE)
   const int La = lines_per_cta(S.na);
@@ -1775,12 +1762,8 @@ extern "C" int hb_spme_recip_noalloc(const float *posq, uint32_t n, const double
       default: k_spread<8><<<hb_div_up(th, 256), 256, 0, s>>>(pq, dbox, na, nb, nc, rho, n); break;
     }
   }
-  if (cube) {
-    HB_TRY(cube_prepare(na));
-    cube_pass(na, rho, v, tw, dbox, bfac, (float)alpha, part, s, true);
-  } else {
-    fft_passes(spme_plan(na, nb, nc), rho, cgrid, v, tw, dbox, bfac, (float)alpha, part, s, false);
-  }
+  if (cube) cube_pass(na, rho, v, tw, dbox, bfac, (float)alpha, part, s, true);
+  else fft_passes(spme_plan(na, nb, nc), rho, cgrid, v, tw, dbox, bfac, (float)alpha, part, s, false);
   if (n > 0) {
     switch (order) {
       case 4: k_gather<4><<<hb_div_up(n, 128), 128, 0, s>>>(pq, v, dbox, na, nb, nc, self_pref, o, n); break;
