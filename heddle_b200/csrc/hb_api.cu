@@ -1720,7 +1720,8 @@ struct hb_batch {
   cudaEvent_t fork = nullptr, t0 = nullptr, t1 = nullptr, pair_done = nullptr;
   cudaGraphExec_t exec = nullptr;
   // 1: one multi-system pair launch for all members (when they share the
-  // pair physics and contexts are distinct); 0 (default, measured faster:
+  // pair physics and contexts are distinct); 0 (default, measured faster, 2,490
+  // against 2,844 us per 10 steps of 12 replicas:
   // members that skip a rebuild start their pair kernels early instead of
   // waiting at the join) = one pair launch per member
   int one_pair_launch = 0;

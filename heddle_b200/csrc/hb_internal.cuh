@@ -570,9 +570,11 @@ int nl_free(hb_forcefield *ff);
 // Rebuild the list.  gated: kernels run only when the status word has the
 // displacement bit set (a device-side decision, no host read).
 int nl_rebuild(hb_forcefield *ff, bool gated, cudaStream_t s);
+// Kernels of one rebuild, launched one by one (eager) or as a graph's body.
 int nl_kernel_count(const hb_forcefield *ff, bool eager);
-// During stream capture: the rebuild as a device-side conditional graph node.
 int nl_displacement_check(hb_forcefield *ff, cudaStream_t s);
+// Check, rebuild where it asks for one (during stream capture as a
+// device-side conditional graph node), positions in tile order.
 int nl_update(hb_forcefield *ff, bool capturing, cudaStream_t s);
 int nl_first_build(hb_forcefield *ff);
 int nl_set_slab(hb_forcefield *ff, uint32_t slab);

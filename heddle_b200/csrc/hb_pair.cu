@@ -25,8 +25,10 @@
 
 // Resident blocks the register budget is cut for.  Force-only: 6 (80
 // registers, no spill) runs the 65,536-water list in 245 us against 248 at 5
-// (96), 258 at 7 (72, 88 B of spill) and 268 at 8 (64, 240 B); with energies
-// or exact sums 5, where the same kernel needs 96 registers.
+// (96), 258 at 7 (72, 88 B of spill) and 268 at 8 (64, 240 B); with scaled
+// exclusions and a switch the same cap spills 72 B.  With energies or exact
+// sums 5, where the kernel needs 96 registers; the multi-system form, which
+// carries its member's pointers, spills 72 B there.
 #define PAIR_MIN_BLOCKS(EV, EXACT, MULTI) ((EV) || (EXACT) || (MULTI) ? 5 : 6)
 
 namespace {
@@ -739,10 +741,16 @@ uint32_t pair_chunk_of(const hb_forcefield *ff) {
 
 // Resident blocks per SM when the caller set none.  With a reciprocal part
 // fewer than fit, so that its chain on the other stream finds SM room beside
-// the persistent blocks: one fewer where whole planes are transformed (graph
-// step of 65,536 waters 414, 392, 453 us at 6, 5, 4; of 8,192 97, 91, 98 us),
-// two fewer where five line passes have to find room (2,000 waters 69, 64,
-// 60 us; 21,952: 209, 204, 196 us)
+// the persistent blocks.  Force-only (6 fit): one fewer where whole planes are
+// transformed (graph step of 65,536 waters 414, 392, 453 us at 6, 5, 4; of
+// 8,192 103, 97, 106 us), two fewer where five line passes have to find room
+// (2,000 waters 69, 64, 60 us; 21,952: 209, 204, 196 us), and the same beside
+// the one-cluster transform, where it makes no difference.  With energies or
+// exact sums (5 fit) one fewer: beside line passes 1,732, 1,609, 1,596,
+// 1,638 us per 20 steps of 1,237 waters with energies at 5, 4, 3, 2 blocks,
+// 1,932, 1,770, 1,791, 1,911 us per relaxation of 2,000 waters, 961, 856, 832,
+// 848 us per 10 exact steps of 13,824 ions.  The multi-system form takes the
+// same four (12 replicas 2,809, 2,844, 2,941 us per 10 steps at 5, 4, 3)
 uint32_t pair_blocks_of(const hb_forcefield *ff, bool wide) {
   if (ff->pair_blocks_per_sm > 0) return (uint32_t)ff->pair_blocks_per_sm;
   const uint32_t fit = wide ? PAIR_MIN_BLOCKS(true, false, false) : PAIR_MIN_BLOCKS(false, false, false);
