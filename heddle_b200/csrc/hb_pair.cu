@@ -105,7 +105,7 @@ __device__ __forceinline__ void red_add(unsigned long long *p, long long v) {
 // the minimum image of the two stored positions, so it is a function of the
 // positions alone, not of the tile the pair was packed into.
 //
-// Bound: instruction issue (about 1,150 warp instructions per entry, of
+// Bound: instruction issue (about 1,190 warp instructions per entry, of
 // which 450 do not depend on the hits) together with shared-memory
 // wavefronts; DRAM and MUFU are far from it.  Against one pair queue per
 // entry with balanced lane runs (1,776 instructions per entry: the queue's
@@ -844,7 +844,11 @@ bool pair_batchable(hb_forcefield *const *ffs, uint32_t n) {
   return a->lj_on || a->coul_on;
 }
 
-// the member table (host-built, copied synchronously: call outside capture)
+// the member table (host-built, copied synchronously: call outside capture).
+// One work-item length for all members, the first one's: with items of all
+// members to take from, the length does not show (12 replicas 2,846, 2,830,
+// 2,838, 2,824 us per 10 steps at 1, 2, 3, 4 entries; with a kernel per member
+// 2,460, 2,416, 2,504, 2,479)
 int pair_batch_table(hb_forcefield *const *ffs, uint32_t n, void *d_table, uint32_t *items_total) {
   std::vector<PairMember> t(n);
   uint32_t item0 = 0;
